@@ -639,6 +639,18 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, int n, uint
       }
     } else {
       if (f.kind == kOpU2) o.code |= op_r_bits(jbit(tbit[f.tq[0]]), jbit(tbit[f.tq[1]]));
+      if (f.kind == kOpDiag) {
+        int k0 = -1, others = 0;
+        for (int k = 0; k < (int)f.mat.size(); ++k)
+          if (f.mat[k] != cd(1)) {
+            others += k0 >= 0;
+            k0 = k;
+          }
+        if (k0 >= 0 && !others) {
+          o.code |= (f.mat[k0] == cd(-1) ? kDiagFlip : kDiagOne) << kDiagShift;
+          o.rmask = k0;
+        }
+      }
       for (const cd& c : f.mat) put(c.real(), c.imag());
     }
     o.nd = f.nd;

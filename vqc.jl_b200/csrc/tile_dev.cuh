@@ -84,6 +84,12 @@ __host__ __device__ constexpr int op_r1(int code) { return ((code >> 6) & 3) | (
 __host__ __device__ constexpr int op_r_bits(int r0, int r1) {
   return ((r0 & 3) << 4) | ((r1 & 3) << 6) | ((r0 >> 2) << 20) | ((r1 >> 2) << 21);
 }
+// Diagonal ops of the packed plan, bits 22-23: what the table holds.  One
+// entry k0 (in rmask) differs from 1 (CPHASE, CCPHASE), or it is exactly -1
+// (CZ): the compiled passes touch only the amplitudes of that entry.
+constexpr int kDiagShift = 22;
+enum { kDiagTable = 0, kDiagOne = 1, kDiagFlip = 2 };
+__host__ __device__ constexpr int diag_class(int code) { return (code >> kDiagShift) & 3; }
 // bits 11-13: one-qubit matrix form; bits 14-15: reduced-matrix entries
 // accumulated; bits 16-18: register control; bit 19: anti-Hermitian projection
 constexpr int kCodeAH = 1 << 19;

@@ -256,6 +256,11 @@ __device__ __forceinline__ void u1_masked(Pk (&v)[NP], Pk (&w)[NP], const u64* c
 #pragma unroll
     for (int g = 0; g < NP / 2; ++g) {
       const int m0 = ((g >> T) << (T + 1)) | (g & ((1 << T) - 1)), m1 = m0 | (1 << T);
+      if (((rmask >> (2 * m0)) & 3) == 3) {  // both lanes: the packed form
+        free_apply<FORM>(v[m0], v[m1], c);
+        if (ADJ) free_apply<FORM, true>(w[m0], w[m1], c);
+        continue;
+      }
       if ((rmask >> (2 * m0)) & 1) {
         scalar_apply<FORM, 0>(v[m0], v[m1], c);
         if (ADJ) scalar_apply<FORM, 0, true>(w[m0], w[m1], c);
@@ -659,6 +664,24 @@ __device__ __forceinline__ void diag_op(Pk (&v)[NP], Pk (&w)[NP], const DevOp* o
     const float2 d = c[idx];
     set_amp(v, j, ccmul(d, amp(v, j)));
     if (ADJ) set_amp(w, j, ccmul(make_float2(d.x, -d.y), amp(w, j)));  // the conjugated cotangent
+  }
+}
+// One pair times a lane-wise complex factor (R + iI; NI = -I).
+__device__ __forceinline__ void phase_pk(Pk& a, u64 R, u64 I, u64 NI) {
+  const u64 ar = a.r, ai = a.i;
+  a.r = fma2(R, ar, mul2(NI, ai));
+  a.i = fma2(R, ai, mul2(I, ar));
+}
+__device__ __forceinline__ void flip_pk(Pk& a, u64 sign) {
+  a.r ^= sign;
+  a.i ^= sign;
+}
+// s8's bin `idx` += (re, im).
+__device__ __forceinline__ void bin_add(float (&s8)[8], uint32_t idx, float re, float im) {
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    s8[2 * b] += idx == (uint32_t)b ? re : 0.f;
+    s8[2 * b + 1] += idx == (uint32_t)b ? im : 0.f;
   }
 }
 // Bins of conj(lam) psi over a diagonal op's (at most 2) qubits -> s8.
