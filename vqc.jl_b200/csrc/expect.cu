@@ -1156,7 +1156,7 @@ static std::string pt_jit_source(bool f32, bool write, bool acc, bool add, bool 
      << "        const int u = (threadIdx.x + kq * NT) << 2;\n"
      << "        const long long g = (long long)nb + shi[u >> CLOW] + (u & ((1 << CLOW) - 1));\n"
      << "        asm volatile(\"prefetch.global.L2 [%0];\" ::\"l\"(ket + g));\n"
-     << (add ? "        asm volatile(\"prefetch.global.L2 [%0];\" ::\"l\"(out + g));\n" : "")
+     << (add && write ? "        asm volatile(\"prefetch.global.L2 [%0];\" ::\"l\"(out + g));\n" : "")
      << "      }\n    }\n"
      << "#pragma unroll 1\n    for (int kq = 0; kq < QPT; ++kq) {\n"
      << "      const int u = (threadIdx.x + kq * NT) << 2;\n"
