@@ -1,0 +1,50 @@
+"""FP64 passes compiled at run time against the interpreted ones.
+
+Both run the same device functions in the same order, so a state, an energy
+and a gradient have the same bits whichever kernel ran: a circuit's first call
+(interpreted, while its passes compile in the background) and its later ones
+agree exactly.  The oracle bounds of both are asserted elsewhere
+(test_gpu_fused.py, test_gpu_tile_forms.py, test_gpu_diag_ops.py with VQC_JIT on
+and off).
+"""
+import numpy as np
+import pytest
+
+import vqcb200 as V
+from helpers import rand_psi
+from test_gpu_fused import random_mixed_circuit
+from vqcb200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [11, 12, 15])
+def test_same_bits(n, monkeypatch):
+    rng = np.random.default_rng(500 + n)
+    c, _ = random_mixed_circuit(rng, n, 80)
+    psi0, target = rand_psi(rng, n), rand_psi(rng, n)
+    got = []
+    for jit in ("off", "on"):
+        monkeypatch.setenv("VQC_JIT", jit)
+        y = c * V.StateVector(psi0)
+        out = y.storage()
+        delta, g, yin = V.back_propagate(V.StateVector(target), c, y)
+        got.append((out, g, delta.storage(), yin.storage()))
+    assert np.array_equal(got[0][0], got[1][0])
+    # (the grid, and with it the order of the sums over CTAs, may differ here)
+    assert np.allclose(got[0][1], got[1][1], rtol=0, atol=1e-12 * np.abs(got[0][1]).max())
+    assert np.array_equal(got[0][2], got[1][2]) and np.array_equal(got[0][3], got[1][3])
+
+
+def test_calls_agree_across_the_compile(monkeypatch):
+    """The default mode at a size that compiles: interpreted, then compiled."""
+    monkeypatch.delenv("VQC_JIT", raising=False)
+    n, layers = 20, 2
+    rng = np.random.default_rng(510)
+    c = W.to_circuit(W.rxyz_crx_spec(n, layers, rng.uniform(0, 2 * np.pi, layers * (4 * n - 1))))
+    H, s = W.to_operator(W.xxz_spec(n, 0.5)), V.StateVector(n)
+    first = V.energy_and_gradient(H, c, s)
+    for _ in range(2):
+        again = V.energy_and_gradient(H, c, s)
+        assert again[0] == first[0]
+        assert np.array_equal(again[1], first[1])

@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 
+#include "cplx.cuh"
 #include "vqc_b200.h"
 
 namespace vqc {
@@ -57,26 +58,6 @@ static int vqc_dbg_read(DebugRecord* out, int reset) {
 #endif
 
 // ----------------------------------------------------------------------------- complex
-template <class R>
-struct CT;
-template <>
-struct CT<float> {
-  using T = float2;
-};
-template <>
-struct CT<double> {
-  using T = double2;
-};
-template <class R>
-using cplx = typename CT<R>::T;
-
-template <class R>
-__host__ __device__ __forceinline__ cplx<R> mkc(R a, R b) {
-  cplx<R> r;
-  r.x = a;
-  r.y = b;
-  return r;
-}
 // a * b
 template <class V>
 __host__ __device__ __forceinline__ V cmul(V a, V b) {

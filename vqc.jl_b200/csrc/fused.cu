@@ -26,10 +26,13 @@
 // the warp, the CTA and the grid, in a fixed order); the host contracts A
 // with D_j = B^dagger dB/dtheta_j of each parameter j of the (merged) block.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <mutex>
+#include <set>
 #include <thread>
 #include <type_traits>
 
@@ -398,45 +401,78 @@ struct Device {
   }
 };
 
-template <class R, int M, bool ADJ>
-static size_t pass_smem(const PassShape& ps) {
-  constexpr int NT = 1 << (M - kRegBits);
-  const size_t npool = (size_t)ps.npool * sizeof(cplx<R>);
-  return tile_bytes<R, M, ADJ>() + (ADJ ? (size_t)ps.nslots * (NT / 32) * 8 * sizeof(double) : 0) +
+// Dynamic shared memory of one pass: the tile(s), the accumulation slots (one
+// row of 8 doubles per warp and slot) and the pass's descriptors.
+static size_t pass_smem(size_t amp, int M, bool adj, const PassShape& ps, int rb = kRegBits) {
+  const size_t nw = (size_t(1) << (M - rb)) / 32, npool = (size_t)ps.npool * amp;
+  return (adj ? 2 : 1) * (amp << M) + (adj ? (size_t)ps.nslots * nw * 8 * sizeof(double) : 0) +
          (ps.packed ? sizeof(DevStageF) : sizeof(DevStage)) * ps.nstages + sizeof(DevOp) * ps.nops +
          ((npool + 15) & ~size_t(15));
 }
 
-// The tile kernel of a pass shape.
-template <class R, int M, bool ADJ>
-static auto tile_kernel(const PassShape& ps) -> decltype(&k_tile<R, M, ADJ, true, false>) {
-  if constexpr (std::is_same<R, float>::value)
-    if (ps.packed) return ps.general ? k_tile<R, M, ADJ, true, true> : k_tile<R, M, ADJ, false, true>;
-  return ps.general ? k_tile<R, M, ADJ, true, false> : k_tile<R, M, ADJ, false, false>;
+// The library's kernel for a pass of that shape (not compiled at run time).
+template <bool ADJ>
+static const void* packed_kernel(int M) {
+  switch (M) {
+    case 12: return (const void*)k_tile_packed<12, ADJ>;
+    case 11: return (const void*)k_tile_packed<11, ADJ>;
+    case 10: return (const void*)k_tile_packed<10, ADJ>;
+    default: return (const void*)k_tile_packed<9, ADJ>;
+  }
+}
+template <class R, bool ADJ>
+static const void* tile_kernel(int M, const PassShape& ps) {
+  return ps.packed ? packed_kernel<ADJ>(M) : (const void*)k_tile<R, ADJ>;
 }
 
-template <class R, int M, bool ADJ>
-static int tile_grid(int device, const PassShape& ps) {
-  constexpr int NT = 1 << (M - kRegBits);
-  const size_t smem = pass_smem<R, M, ADJ>(ps);
-  auto kfun = tile_kernel<R, M, ADJ>(ps);
-  cudaFuncSetAttribute(kfun, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024));
+// Lets kernel k use all the shared memory a block may have, once per device
+// and kernel: a limit set per launch could be lowered by another thread between
+// its setting and its launch (the serving loop's planners size the same kernels).
+static int allow_smem(int device, const void* k) {
+  static std::mutex mu;
+  static std::set<std::pair<int, const void*>> done;
+  std::lock_guard<std::mutex> lk(mu);
+  if (done.count({device, k})) return VQC_OK;
+  cudaFuncAttributes fa;
+  VQC_CK(cudaFuncGetAttributes(&fa, k));
+  VQC_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              device_info(device).max_smem_optin - (int)fa.sharedSizeBytes));
+  done.insert({device, k});
+  return VQC_OK;
+}
+
+// Resident CTAs of a tile kernel over the whole device.
+static int kernel_grid(int device, const void* k, int nt, size_t smem) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfun, NT, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+  if (allow_smem(device, k) || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, smem) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    per_sm = 1;
+  }
   return device_info(device).sms * per_sm;
 }
 
 template <class R, int M, bool ADJ>
-static int launch_tile(vqc_state h, void* psi, void* lam, const DevPass* dp, const void* ds, const DevOp* dops,
-                       const void* pool, double* partials, int grid, const PassShape& ps, double flops) {
-  constexpr int NT = 1 << (M - kRegBits);
-  const size_t smem = pass_smem<R, M, ADJ>(ps);
-  auto kfun = tile_kernel<R, M, ADJ>(ps);
-  VQC_CK(cudaFuncSetAttribute(kfun, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024)));
+static int launch_tile(vqc_state h, const TileItem& item, const PassShape& ps, double flops) {
+  const size_t smem = pass_smem(sizeof(cplx<R>), M, ADJ, ps);
+  const void* k = tile_kernel<R, ADJ>(M, ps);
+  if (int rc = allow_smem(h->device, k)) return rc;
   ProfScope prof(h->stream, ADJ ? "tile_adjoint" : "tile_forward",
                  (double)(ADJ ? 4 : 2) * h->size() * sizeof(cplx<R>), flops);
-  kfun<<<grid, NT, smem, h->stream>>>((cplx<R>*)psi, (cplx<R>*)lam, dp, ds, dops, (const cplx<R>*)pool, partials);
-  VQC_CK(cudaGetLastError());
+  void* args[] = {const_cast<TileItem*>(&item)};
+  VQC_CK(cudaLaunchKernel(k, dim3(item.ncta), dim3(1 << (M - kRegBits)), args, smem, h->stream));
+  return VQC_OK;
+}
+
+// A compiled FP64 pass; its matrices (host copy) are the kernel's second parameter.
+template <int M, bool ADJ>
+static int launch_tile64(vqc_state h, const void* k, const TileItem& item, const PassShape& ps, const void* host_pool,
+                         double flops) {
+  const size_t smem = pass_smem(sizeof(double2), M, ADJ, ps);
+  if (int rc = allow_smem(h->device, k)) return rc;
+  ProfScope prof(h->stream, ADJ ? "tile_adjoint" : "tile_forward",
+                 (double)(ADJ ? 4 : 2) * h->size() * sizeof(double2), flops);
+  void* args[] = {const_cast<TileItem*>(&item), const_cast<void*>(host_pool)};
+  VQC_CK(cudaLaunchKernel(k, dim3(item.ncta), dim3(1 << (M - kRegBits)), args, smem, h->stream));
   return VQC_OK;
 }
 
@@ -480,18 +516,28 @@ static bool acc_anti_hermitian(const FOp& f) {
   return !f.grads.empty();
 }
 
+// A diagonal gate with one entry that is not 1: that entry, else -1.
+static int single_entry(const FOp& f) {
+  int k0 = -1;
+  for (int k = 0; k < (int)f.mat.size(); ++k)
+    if (f.mat[k] != cd(1)) {
+      if (k0 >= 0) return -1;
+      k0 = k;
+    }
+  return k0;
+}
+
 // FMA-pipe lane operations (fused multiply-adds, multiplies, adds) of one pass
 // over the whole state of n qubits, as the tile bodies implement its ops: a
 // one-qubit op costs per amplitude pair and state 16 (general form), 8
 // (RX-like, real, diagonal) or 0 (swap), and in the reverse sweep its
-// reduced-matrix accumulation 16 / 8 per pair (12 / 8 / 4 for the FP32
+// reduced-matrix accumulation 16 / 8 per pair (12 / 8 / 4 for the
 // anti-Hermitian projection); a two-qubit op 64 per amplitude quad and state;
-// a diagonal op 4 per amplitude and state (6 more for its accumulation).
-// Controls scale by the fraction of amplitudes they enable.  The classic body
-// runs every forward one-qubit op in the general form, and in the reverse
-// sweep the RX-like form or the general one.  The numerator of the compute
-// roofline (vqc_fma_peak is the denominator).
-static double pass_fma_ops(const PlanPass& p, int n, bool adj, bool packed) {
+// a diagonal op 4 per state and amplitude that an entry other than 1 touches
+// (a flip of sign none), 4 more for its accumulation.  Controls scale by the
+// fraction of amplitudes they enable.  The numerator of the compute roofline
+// (vqc_fma_peak is the denominator).
+static double pass_fma_ops(const PlanPass& p, int n, bool adj) {
   const double pairs = std::ldexp(1.0, n - 1), amps = std::ldexp(1.0, n);
   const int nst = adj ? 2 : 1;
   static const int per_pair[5] = {16, 8, 8, 8, 0};  // by kForm*
@@ -499,12 +545,10 @@ static double pass_fma_ops(const PlanPass& p, int n, bool adj, bool packed) {
   for (const FOp& f : p.ops) {
     const double act = std::ldexp(1.0, -popc64(f.cmask));
     if (f.kind == kOpU1) {
-      int form = u1_form(f.mat);
-      if (!packed) form = adj ? (form == kFormRI ? kFormRI : kFormGen) : kFormGen;
-      double o = (double)per_pair[form] * nst;
+      double o = (double)per_pair[u1_form(f.mat)] * nst;
       if (adj && f.acc) {
         const int k = acc_kind(f);
-        if (packed && acc_anti_hermitian(f))
+        if (acc_anti_hermitian(f))
           o += k == kAccFull ? 12 : (k == kAccOff ? 8 : 4);
         else
           o += k == kAccFull ? 16 : 8;
@@ -513,10 +557,52 @@ static double pass_fma_ops(const PlanPass& p, int n, bool adj, bool packed) {
     } else if (f.kind == kOpU2) {
       ops += 64.0 * nst * (amps / 4) * act;
     } else if (f.kind == kOpDiag) {
-      ops += 4.0 * nst * amps + (adj && f.acc ? 6.0 * amps : 0.0);
+      const int k0 = single_entry(f);
+      const double touched = k0 < 0 ? 1.0 : (f.mat[k0] == cd(-1) ? 0.0 : std::ldexp(1.0, -f.nd));
+      ops += 4.0 * nst * amps * touched + (adj && f.acc ? 4.0 * amps : 0.0);
     }
   }
   return ops;
+}
+
+// The controls of an op by place: qubits outside the tile (one test per tile),
+// thread bits (one test per op), register bits (rc, and the amplitudes they
+// enable in rmask).
+static void place_controls(DevOp& o, uint64_t cmask, uint64_t cval, int n, uint64_t tile_mask,
+                           std::map<int, int>& tbit, const std::vector<int>& rs, std::vector<std::pair<int, int>>& rc) {
+  for (int q = 0; q < n; ++q) {
+    if (!(cmask >> q & 1)) continue;
+    const int v = (int)(cval >> q & 1);
+    if (!(tile_mask >> q & 1)) {
+      o.gmask |= 1ull << q;
+      if (v) o.gval |= 1ull << q;
+      continue;
+    }
+    const int b = tbit[q], j = (int)(std::find(rs.begin(), rs.end(), b) - rs.begin());
+    if (j < (int)rs.size()) {
+      rc.push_back({j, v});
+    } else {
+      o.cmask |= 1u << b;
+      if (v) o.cval |= 1u << b;
+    }
+  }
+  uint32_t rmask = 0;
+  for (uint32_t j = 0; j < (1u << rs.size()); ++j) {
+    bool ok = true;
+    for (auto& c : rc) ok = ok && ((int)(j >> c.first & 1) == c.second);
+    if (ok) rmask |= 1u << j;
+  }
+  o.rmask = (int32_t)rmask;
+  if (o.cmask) o.code |= kCodeCtl;
+  if (o.gmask) o.code |= kCodeGCtl;
+}
+
+// Tile bits of the warp index (thread bits 5 and up) in a stage's layout.
+static uint32_t warp_bits(const PlanStage& st, int M) {
+  uint32_t m = 0;
+  for (int b = 0, i = 0; b < M; ++b)
+    if (std::find(st.rs.begin(), st.rs.end(), b) == st.rs.end() && i++ >= 5) m |= 1u << b;
+  return m;
 }
 
 // One stage of the FP32 (packed) tile body: its DevStageF tables, its ops
@@ -571,33 +657,9 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, int n, uint
     o.code = f.kind;
     o.slot = -1;
     std::vector<std::pair<int, int>> rc;  // register controls: (j-bit, value)
-    for (int q = 0; q < n; ++q) {
-      if (!(f.cmask >> q & 1)) continue;
-      const int v = (int)(f.cval >> q & 1);
-      if (tile_mask >> q & 1) {
-        const int b = tbit[q];
-        if (rsmask >> b & 1) {
-          rc.push_back({jbit(b), v});
-        } else {
-          o.cmask |= 1u << b;
-          if (v) o.cval |= 1u << b;
-        }
-      } else {
-        o.gmask |= 1ull << q;
-        if (v) o.gval |= 1ull << q;
-      }
-    }
-    uint32_t rmask = 0;
-    for (int j = 0; j < na; ++j) {
-      bool ok = true;
-      for (auto& c : rc) ok = ok && ((j >> c.first & 1) == c.second);
-      if (ok) rmask |= 1u << j;
-    }
-    o.rmask = (int32_t)rmask;
+    place_controls(o, f.cmask, f.cval, n, tile_mask, tbit, rs, rc);
     int rctl = 0;
     if (!rc.empty()) rctl = (rc.size() == 1 && rc[0].second == 1) ? rc[0].first + 1 : 7;
-    if (o.cmask) o.code |= kCodeCtl;
-    if (o.gmask) o.code |= kCodeGCtl;
     while (pool.size() % 2) put(0, 0);  // each op's block starts on 16 bytes
     o.mat = (int)(pool.size() - pool_begin);
     if (f.kind == kOpU1) {
@@ -640,13 +702,8 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, int n, uint
     } else {
       if (f.kind == kOpU2) o.code |= op_r_bits(jbit(tbit[f.tq[0]]), jbit(tbit[f.tq[1]]));
       if (f.kind == kOpDiag) {
-        int k0 = -1, others = 0;
-        for (int k = 0; k < (int)f.mat.size(); ++k)
-          if (f.mat[k] != cd(1)) {
-            others += k0 >= 0;
-            k0 = k;
-          }
-        if (k0 >= 0 && !others) {
+        const int k0 = single_entry(f);
+        if (k0 >= 0) {
           o.code |= (f.mat[k0] == cd(-1) ? kDiagFlip : kDiagOne) << kDiagShift;
           o.rmask = k0;
         }
@@ -720,22 +777,33 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
       DevStage s{};
       uint32_t rsmask = 0;
       for (int b : st.rs) rsmask |= 1u << b;
+      std::vector<int> thr;
+      for (int b = 0; b < M; ++b)
+        if (!(rsmask >> b & 1)) thr.push_back(b);
+      auto gq = [&](uint32_t t) {
+        int64_t g = 0;
+        for (int b = 0; b < M; ++b)
+          if (t >> b & 1) g |= int64_t(1) << p.tile_q[b];
+        return g;
+      };
       for (int j = 0; j < 16; ++j) {
         uint32_t t = 0;
         for (int i = 0; i < kRegBits; ++i)
           if (j >> i & 1) t |= 1u << st.rs[i];
         s.dep[j] = t;
+        s.swm[j] = Swz<R>::f(t);
+        s.gdep[j] = gq(t);
       }
-      s.thr_mask = ((1u << M) - 1) & ~rsmask;
-      s.gthr_mask = 0;
-      for (int b = 0; b < M; ++b)
-        if (s.thr_mask >> b & 1) s.gthr_mask |= 1ull << p.tile_q[b];
-      for (int j = 0; j < 16; ++j) {
-        int64_t g = 0;
-        for (int b = 0; b < M; ++b)
-          if (s.dep[j] >> b & 1) g |= int64_t(1) << p.tile_q[b];
-        s.gdep[j] = g;
-      }
+      for (int k = 0; k < 2; ++k)
+        for (int nib = 0; nib < 16; ++nib) {
+          uint32_t t = 0;
+          for (int i = 0; i < 4; ++i)
+            if ((nib >> i & 1) && 4 * k + i < (int)thr.size()) t |= 1u << thr[4 * k + i];
+          s.thr[k][nib] = t;
+          s.swt[k][nib] = Swz<R>::f(t);
+          s.gthr[k][nib] = gq(t);
+        }
+      s.cta = warp_bits(st, M) != warp_bits(p.stages[(&st - p.stages.data() + 1) % p.stages.size()], M);
       s.op_begin = (int)dops.size();
       for (int oi : st.ops) {
         const FOp& f = p.ops[oi];
@@ -743,27 +811,47 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
         o.code = f.kind;
         o.slot = -1;
         auto slot_of = [&](int b) { return (int)(std::find(st.rs.begin(), st.rs.end(), b) - st.rs.begin()); };
+        // a phase on one entry of a diagonal gate is an op behind controls
+        const int k0 = f.kind == kOpDiag ? single_entry(f) : -1;
+        uint64_t cm = f.cmask, cv = f.cval;
+        for (int i = 0; k0 >= 0 && i < f.nd; ++i) {
+          cm |= 1ull << f.dq[i];
+          if (k0 >> i & 1) cv |= 1ull << f.dq[i];
+        }
+        std::vector<std::pair<int, int>> rc;
+        place_controls(o, cm, cv, n, tile_mask, tbit, st.rs, rc);
+        int sel = k0 < 0 ? kSelDiag : (f.mat[k0] == cd(-1) ? kSelFlip : kSelPhase);
         if (f.kind == kOpU1) {
-          o.code |= slot_of(tbit[f.tq[0]]) << 4;
-          o.code |= u1_form(f.mat) << 11;
-          if (ADJ && f.acc) o.code |= acc_kind(f) << 14;
+          const int r = slot_of(tbit[f.tq[0]]), form = u1_form(f.mat);
+          sel = kSelU1 + (r | (rc.empty() ? 0 : 4) | form << 3);
+          if (ADJ && f.acc) o.code |= (acc_kind(f) << 14) | (acc_anti_hermitian(f) ? kCodeAH : 0);
         }
-        if (f.kind == kOpU2) o.code |= (slot_of(tbit[f.tq[0]]) << 4) | (slot_of(tbit[f.tq[1]]) << 6);
-        for (int q = 0; q < n; ++q) {
-          if (!(f.cmask >> q & 1)) continue;
-          const bool v = f.cval >> q & 1;
-          if (tile_mask >> q & 1) {
-            o.cmask |= 1u << tbit[q];
-            if (v) o.cval |= 1u << tbit[q];
-          } else {
-            o.gmask |= 1ull << q;
-            if (v) o.gval |= 1ull << q;
+        if (f.kind == kOpU2) sel = kSelU2 + slot_of(tbit[f.tq[0]]) * 4 + slot_of(tbit[f.tq[1]]);
+        if (k0 >= 0) o.code = (o.code & ~15) | kOpPhase;
+        // the thread's amplitudes it acts on, for the interpreted body
+        uint32_t held = 0;
+        int nfree = 0;
+        if (f.kind == kOpU1 || f.kind == kOpU2)
+          for (int i = 0; i < (f.kind == kOpU1 ? 1 : 2); ++i) {
+            const int r = slot_of(tbit[f.tq[i]]);
+            held |= 1u << r;
+            o.target[i] = (uint16_t)s.swm[1 << r];
           }
+        for (auto& c : rc) {
+          held |= 1u << c.first;
+          if (c.second) o.first ^= (uint16_t)s.swm[1 << c.first];
         }
-        if (o.cmask) o.code |= kCodeCtl;
-        if (o.gmask) o.code |= kCodeGCtl;
+        for (int r = 0; r < kRegBits; ++r)
+          if (!(held >> r & 1)) {
+            if (nfree < 3) o.step[nfree] = (uint16_t)s.swm[1 << r];
+            ++nfree;
+          }
+        o.code |= sel << kSelShift | nfree << 16;
         o.mat = (int)(pool.size() - pool_begin);
-        for (const cd& c : f.mat) pool.push_back(mkc<R>((R)c.real(), (R)c.imag()));
+        if (k0 >= 0)
+          pool.push_back(mkc<R>((R)f.mat[k0].real(), (R)f.mat[k0].imag()));
+        else
+          for (const cd& c : f.mat) pool.push_back(mkc<R>((R)c.real(), (R)c.imag()));
         o.nd = f.nd;
         for (int i = 0; i < 5; ++i) {
           o.dbit[i] = -1;
@@ -778,15 +866,18 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
         if (ADJ && f.acc) {
           o.slot = slot++;
           if (f.kind == kOpDiag) {
-            // the accumulation runs as its own op right after the diagonal
+            // the accumulation runs as its own op right after the diagonal, over
+            // every bin (no controls)
             dops.push_back(o);
             DevOp a = o;
-            a.code = (a.code & ~15) | kOpAccD;
+            a.code = kOpAccD | kCodeAcc | (kSelAccD << kSelShift);
+            a.cmask = a.cval = 0;
+            a.gmask = a.gval = 0;
             dops.push_back(a);
             if (accs) accs->push_back(AccRef{row + o.slot, f});
             continue;
           }
-          if (accs) accs->push_back(AccRef{row + o.slot, f});
+          if (accs) accs->push_back(AccRef{row + o.slot, f, (o.code & kCodeAH) != 0});
           o.code |= kCodeAcc;
         }
         dops.push_back(o);
@@ -807,13 +898,10 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
     locs[pi].shape.nstages = (int)p.stages.size();
     locs[pi].shape.nops = P.nops;
     locs[pi].shape.npool = P.npool;
-    locs[pi].shape.general = false;
-    for (const DevOp& o : dops)
-      if ((o.code & 15) != kOpU1) locs[pi].shape.general = true;
     locs[pi].row0 = row;
     row += slot;
     locs[pi].nslots = slot;
-    locs[pi].fma_ops = pass_fma_ops(p, n, ADJ, packed);
+    locs[pi].fma_ops = pass_fma_ops(p, n, ADJ);
     // stage indices are local to this pass's stage array
     P.stage_begin = 0;
     P.stage_end = (int)p.stages.size();
@@ -850,25 +938,12 @@ static void note_plan(bool adj, const std::vector<PlanPass>& passes) {
 }
 
 template <int M, bool ADJ>
-static int jit_grid(int device, const void* k, const PassShape& ps, int rb = kRegBits) {
-  const int NT = 1 << (M - rb);
-  const size_t smem = pass_smem<float, M, ADJ>(ps) + jit_extra_smem(ADJ, M, rb);
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024));
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, smem) != cudaSuccess || per_sm < 1) {
-    cudaGetLastError();
-    per_sm = 1;
-  }
-  return device_info(device).sms * per_sm;
-}
-
-template <int M, bool ADJ>
 static int launch_tile_jit(vqc_state h, const void* k, void* psi, void* lam, const DevPass* dp, const void* ds,
                            const DevOp* dops, const void* pool, double* partials, int grid, const PassShape& ps,
                            const void* host_pool, double flops, int rb = kRegBits) {
   const int NT = 1 << (M - rb);
-  const size_t smem = pass_smem<float, M, ADJ>(ps) + jit_extra_smem(ADJ, M, rb);
-  VQC_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024)));
+  const size_t smem = pass_smem(sizeof(float2), M, ADJ, ps) + jit_extra_smem(ADJ, M, rb);
+  if (int rc = allow_smem(h->device, k)) return rc;
   ProfScope prof(h->stream, ADJ ? "tile_adjoint" : "tile_forward", (double)(ADJ ? 4 : 2) * h->size() * sizeof(float2),
                  flops);
   // the last parameter is the pass's matrix pool by value (host copy)
@@ -886,6 +961,15 @@ static bool use_jit(const vqc_state h) {
 // The packed FP32 plan layout: for the compiled passes, or forced with
 // VQC_JIT=interp (the packed interpreter, the compiled kernels' fallback).
 static bool use_packed(const vqc_state h) { return h->dtype == VQC_C64 && (use_jit(h) || jit_mode() == 3); }
+// Compiled FP64 passes: states of at least 2^20 amplitudes (auto), all (on).
+static bool use_jit64(const vqc_state h) {
+  const int mode = jit_mode();
+  return h->dtype == VQC_C128 && (mode == 1 || (mode == 2 && h->nq >= 20)) && jit_available();
+}
+static uint64_t new_call() {
+  static std::atomic<uint64_t> n{0};
+  return ++n;
+}
 // VQC_JIT_WIDE=1: compiled forward passes with 32 amplitudes per thread (four
 // free register bits per stage: 3.0 instead of 3.8 stages per pass on the
 // headline circuit).  Off by default: measured slower at 2^26 amplitudes
@@ -911,7 +995,8 @@ static size_t op_bytes_bound(const PlanPass& p) {
 // chunks of one sweep can be uploaded while these passes run.
 template <class R, int M, bool ADJ>
 static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& passes, const std::vector<GateSpec>& specs,
-                    std::vector<AccRef>* accs, double* rows_dev, size_t op_off = 0, size_t* op_used = nullptr) {
+                    std::vector<AccRef>* accs, double* rows_dev, uint64_t call, size_t op_off = 0,
+                    size_t* op_used = nullptr) {
   const int n = h->nq;
   SerialPlan sp;
   const bool packed = use_packed(h);
@@ -950,15 +1035,27 @@ static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& pa
       }
     }
   }
+  if constexpr (std::is_same<R, double>::value) {
+    if (use_jit64(h)) {
+      std::vector<JitPassRef64> refs(passes.size());
+      for (size_t pi = 0; pi < passes.size(); ++pi)
+        if (!sp.locs[pi].standalone)
+          refs[pi] = JitPassRef64{(const DevStage*)(sp.buf.data() + sp.locs[pi].stages), sp.locs[pi].shape.nstages,
+                                  (const DevOp*)(sp.buf.data() + sp.locs[pi].ops), sp.locs[pi].shape.npool};
+      jit_pass_kernels64(M, ADJ, refs, jk, call, jit_mode() == 1);
+    }
+  }
   const std::vector<PassLoc>& locs = sp.locs;
   const size_t pool_off = sp.pool_off;
   std::vector<int> grids(passes.size(), 0);
   for (size_t pi = 0; pi < passes.size(); ++pi) {
     if (locs[pi].standalone) continue;
-    int g = 0;
-    if constexpr (std::is_same<R, float>::value)
-      if (jk[pi]) g = jit_grid<M, ADJ>(h->device, jk[pi], locs[pi].shape, rb);
-    if (!g) g = tile_grid<R, M, ADJ>(h->device, locs[pi].shape);
+    const size_t smem = pass_smem(sizeof(cplx<R>), M, ADJ, locs[pi].shape);
+    int g = jk[pi] ? kernel_grid(h->device, jk[pi], 1 << (M - rb), smem + jit_extra_smem(ADJ, M, rb))
+                         : kernel_grid(h->device, tile_kernel<R, ADJ>(M, locs[pi].shape), 1 << (M - kRegBits), smem);
+    // the CTAs' partial sums group alike in both kernels of an FP64 pass
+    if constexpr (ADJ && std::is_same<R, double>::value)
+      if (use_jit64(h)) g = device_info(h->device).sms * jit_min_blocks64(true);
     grids[pi] = (int)std::min<int64_t>(g, locs[pi].ntiles);
   }
   // partial sums scratch: one row of 8 doubles per (CTA, slot) of every pass,
@@ -1018,15 +1115,21 @@ static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& pa
     const void* ds = (const void*)(base + locs[pi].stages);
     const DevOp* dops = (const DevOp*)(base + locs[pi].ops);
     const void* dpool = base + pool_off + locs[pi].pool_begin * sizeof(cplx<R>);
+    TileItem it{psi, lam, dp, ds, dops, dpool, pp, locs[pi].ntiles, grid, M, DevPass()};
+    std::memcpy(&it.p, sp.buf.data() + locs[pi].pass, sizeof(DevPass));
     if (jk[pi]) {
+      if constexpr (std::is_same<R, double>::value)
+        if ((rc = launch_tile64<M, ADJ>(h, jk[pi], it, locs[pi].shape,
+                                        sp.buf.data() + pool_off + locs[pi].pool_begin * sizeof(double2),
+                                        2.0 * locs[pi].fma_ops)))
+          return rc;
       if constexpr (std::is_same<R, float>::value)
         if ((rc = launch_tile_jit<M, ADJ>(h, jk[pi], psi, lam, dp, ds, dops, dpool, pp, grid,
                                           locs[pi].shape,
                                           sp.buf.data() + pool_off + locs[pi].pool_begin * sizeof(float2),
                                           2.0 * locs[pi].fma_ops, rb)))
           return rc;
-    } else if ((rc = launch_tile<R, M, ADJ>(h, psi, lam, dp, ds, dops, dpool, pp, grid, locs[pi].shape,
-                                            2.0 * locs[pi].fma_ops))) {
+    } else if ((rc = launch_tile<R, M, ADJ>(h, it, locs[pi].shape, 2.0 * locs[pi].fma_ops))) {
       return rc;
     }
   }
@@ -1065,9 +1168,10 @@ static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const do
       return analyze_gate(h->nq, gates[bad[t]].nq, gates[bad[t]].pos, mats + gates[bad[t]].mat, false, specs[bad[t]]);
   std::vector<PlanPass> passes;
   plan_passes(h->nq, tile_config(h->dtype, h->nq), false, items, passes);
+  const uint64_t call = new_call();
   const char* pc = std::getenv("VQC_PLAN_CHUNKS");  // 0: one serialisation for the whole sweep
   if (passes.size() < 4 || (pc && *pc && std::atoi(pc) == 0))
-    return run_plan<R, M, false>(h, h->d, nullptr, passes, specs, nullptr, nullptr);
+    return run_plan<R, M, false>(h, h->d, nullptr, passes, specs, nullptr, nullptr, call);
   // Serialised and launched in chunks of 1, 2, 4, ... passes: the host plans
   // the next chunk while the device runs the previous ones, instead of the
   // device waiting for the whole sweep's descriptors (about 1.5 ms for 2,000
@@ -1082,7 +1186,7 @@ static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const do
     std::vector<PlanPass> chunk(std::make_move_iterator(passes.begin() + first),
                                 std::make_move_iterator(passes.begin() + last));
     size_t used = 0;
-    if ((rc = run_plan<R, M, false>(h, h->d, nullptr, chunk, specs, nullptr, nullptr, off, &used))) return rc;
+    if ((rc = run_plan<R, M, false>(h, h->d, nullptr, chunk, specs, nullptr, nullptr, call, off, &used))) return rc;
     off = (off + used + 255) & ~size_t(255);
   }
   return VQC_OK;
@@ -1175,6 +1279,7 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
     h->accbuf_rows = rows32;
   }
   // run pass by pass so that standalone gates with parameters see the right states
+  const uint64_t call = new_call();
   std::vector<PlanPass> one(1);
   int row_base = 0;
   for (size_t pi = 0; pi < passes.size(); ++pi) {
@@ -1195,7 +1300,7 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
     std::vector<PlanPass> group;
     while (pj < passes.size() && !passes[pj].standalone) group.push_back(std::move(passes[pj++]));
     std::vector<AccRef> gaccs;
-    int rc = run_plan<R, M, true>(h, y, lam, group, specs, &gaccs, h->accbuf + (size_t)row_base * 8);
+    int rc = run_plan<R, M, true>(h, y, lam, group, specs, &gaccs, h->accbuf + (size_t)row_base * 8, call);
     if (rc) return rc;
     for (auto& a : gaccs) {
       a.row += row_base;
@@ -1370,88 +1475,50 @@ void serve_compile_plan(const ReqPlan& packed, bool want_grad) {
   if (want_grad) plan_kernels(packed.M, true, packed.adj, ks, true);
 }
 
-// Shared memory of a compiled FP32 pass of shape ps (the formula of pass_smem).
-static size_t jit_pass_smem(int M, bool adj, const PassShape& ps) {
-  const size_t nt = size_t(1) << (M - kRegBits);
-  const size_t npool = (size_t)ps.npool * sizeof(float2);
-  return (adj ? 2 : 1) * (size_t(1) << M) * sizeof(float2) + (adj ? (size_t)ps.nslots * (nt / 32) * 8 * sizeof(double) : 0) +
-         sizeof(DevStageF) * ps.nstages + sizeof(DevOp) * ps.nops + ((npool + 15) & ~size_t(15));
-}
-
 int serve_jit_gridx(int M, bool adj, const std::vector<const void*>& ks, const SerialPlan& sp, int64_t ntiles,
                     int device) {
-  int per_sm = 1 << 20;
-  for (size_t i = 0; i < ks.size(); ++i) {
-    const size_t smem = jit_pass_smem(M, adj, sp.locs[i].shape);
-    cudaFuncSetAttribute(ks[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024));
-    int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, ks[i], 1 << (M - kRegBits), smem) != cudaSuccess || b < 1) {
-      cudaGetLastError();
-      b = 1;
-    }
-    per_sm = std::min(per_sm, b);
-  }
-  if (ks.empty()) per_sm = 1;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)device_info(device).sms * per_sm));
+  int grid = ks.empty() ? device_info(device).sms : 1 << 30;
+  for (size_t i = 0; i < ks.size(); ++i)
+    grid = std::min(grid, kernel_grid(device, ks[i], 1 << (M - kRegBits),
+                                      pass_smem(sizeof(float2), M, adj, sp.locs[i].shape)));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, grid));
 }
 
 int serve_launch_jit(int M, bool adj, const void* kernel, const TileItem* d_items, int nitems, int gridx,
                      const PassShape& maxs, cudaStream_t stream) {
-  const size_t smem = jit_pass_smem(M, adj, maxs);
-  VQC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)std::max<size_t>(smem, 48 * 1024)));
+  const size_t smem = pass_smem(sizeof(float2), M, adj, maxs);
+  int device = 0;
+  VQC_CK(cudaGetDevice(&device));
+  if (int rc = allow_smem(device, kernel)) return rc;
   ProfScope prof(stream, adj ? "serve_tile_adjoint" : "serve_tile_forward", 0);
   void* args[] = {(void*)&d_items};
   VQC_CK(cudaLaunchKernel(kernel, dim3(gridx, nitems), dim3(1 << (M - kRegBits)), args, smem, stream));
   return VQC_OK;
 }
 
-template <class R, int M, bool ADJ>
-static int grid_x_tm(const PassShape& maxs, int64_t max_ntiles, int device) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>(max_ntiles, tile_grid<R, M, ADJ>(device, maxs)));
+static const void* batch_kernel(int dtype, bool adj) {
+  if (dtype == VQC_C64) return adj ? (const void*)k_tile_batch<float, true> : (const void*)k_tile_batch<float, false>;
+  return adj ? (const void*)k_tile_batch<double, true> : (const void*)k_tile_batch<double, false>;
 }
-
-template <class R, int M, bool ADJ>
-static int launch_batch_tm(const TileItem* d_items, int nitems, int gridx, const PassShape& maxs,
-                           cudaStream_t stream) {
-  constexpr int NT = 1 << (M - kRegBits);
-  const size_t smem = pass_smem<R, M, ADJ>(maxs);
-  auto kfun = k_tile_batch<R, M, ADJ>;
-  VQC_CK(cudaFuncSetAttribute(kfun, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 48 * 1024)));
-  ProfScope prof(stream, ADJ ? "serve_tile_adjoint" : "serve_tile_forward", 0);
-  kfun<<<dim3(gridx, nitems), NT, smem, stream>>>(d_items);
-  VQC_CK(cudaGetLastError());
-  return VQC_OK;
-}
-
-#define VQC_TILE_SWITCH(FN, ...)                                         \
-  switch (M + (dtype == VQC_C64 ? 0 : 100) + (adj ? 1000 : 0)) {          \
-    case 12: return FN<float, 12, false>(__VA_ARGS__);                    \
-    case 11: return FN<float, 11, false>(__VA_ARGS__);                    \
-    case 10: return FN<float, 10, false>(__VA_ARGS__);                    \
-    case 9: return FN<float, 9, false>(__VA_ARGS__);                      \
-    case 1012: return FN<float, 12, true>(__VA_ARGS__);                   \
-    case 1011: return FN<float, 11, true>(__VA_ARGS__);                   \
-    case 1010: return FN<float, 10, true>(__VA_ARGS__);                   \
-    case 1009: return FN<float, 9, true>(__VA_ARGS__);                    \
-    case 111: return FN<double, 11, false>(__VA_ARGS__);                  \
-    case 110: return FN<double, 10, false>(__VA_ARGS__);                  \
-    case 109: return FN<double, 9, false>(__VA_ARGS__);                   \
-    case 1111: return FN<double, 11, true>(__VA_ARGS__);                  \
-    case 1110: return FN<double, 10, true>(__VA_ARGS__);                  \
-    case 1109: return FN<double, 9, true>(__VA_ARGS__);                   \
-    default: return fail(VQC_ERR_ARG, "no tile kernel for this size");   \
-  }
 
 int serve_tile_gridx(int dtype, int M, bool adj, const PassShape& maxs, int64_t max_ntiles, int device) {
-  VQC_TILE_SWITCH(grid_x_tm, maxs, max_ntiles, device)
+  const size_t smem = pass_smem(dtype == VQC_C64 ? 8 : 16, M, adj, maxs);
+  const int g = kernel_grid(device, batch_kernel(dtype, adj), 1 << (M - kRegBits), smem);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(max_ntiles, g));
 }
 
 int serve_launch_tiles(int dtype, int M, bool adj, const TileItem* d_items, int nitems, int gridx,
                        const PassShape& maxs, cudaStream_t stream) {
-  VQC_TILE_SWITCH(launch_batch_tm, d_items, nitems, gridx, maxs, stream)
+  const size_t smem = pass_smem(dtype == VQC_C64 ? 8 : 16, M, adj, maxs);
+  const void* k = batch_kernel(dtype, adj);
+  int device = 0;
+  VQC_CK(cudaGetDevice(&device));
+  if (int rc = allow_smem(device, k)) return rc;
+  ProfScope prof(stream, adj ? "serve_tile_adjoint" : "serve_tile_forward", 0);
+  void* args[] = {(void*)&d_items};
+  VQC_CK(cudaLaunchKernel(k, dim3(gridx, nitems), dim3(1 << (M - kRegBits)), args, smem, stream));
+  return VQC_OK;
 }
-#undef VQC_TILE_SWITCH
 
 int serve_launch_reduce(const RedItem* d_items, int nitems, int maxslots, cudaStream_t stream) {
   if (nitems == 0 || maxslots == 0) return VQC_OK;

@@ -23,9 +23,12 @@
 #include <nvrtc.h>
 
 #include <algorithm>
+#include <condition_variable>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <set>
 #include <sstream>
@@ -37,7 +40,7 @@ namespace vqc {
 
 namespace {
 
-#include "jit_src.inc"  // kJitTileDev, kJitTileF32: the device headers as text (generated at build time)
+#include "jit_src.inc"  // kJitTileDev, kJitTileF32, ...: the device headers as text (generated at build time)
 
 struct Nvrtc {
   bool ok = false;
@@ -96,9 +99,9 @@ int env_int(const char* name, int dflt) {
 bool compile_one(const std::string& src, std::vector<char>& cubin, std::string& log) {
   const Nvrtc& nv = nvrtc();
   nvrtcProgram prog;
-  const char* hdrs[2] = {kJitTileDev, kJitTileF32};
-  const char* names[2] = {"tile_dev.cuh", "tile_f32.cuh"};
-  if (nv.create(&prog, src.c_str(), "vqc_pass.cu", 2, hdrs, names) != NVRTC_SUCCESS) {
+  const char* hdrs[4] = {kJitTileDev, kJitTileF32, kJitCplx, kJitTileOps};
+  const char* names[4] = {"tile_dev.cuh", "tile_f32.cuh", "cplx.cuh", "tile_ops.cuh"};
+  if (nv.create(&prog, src.c_str(), "vqc_pass.cu", 4, hdrs, names) != NVRTC_SUCCESS) {
     log = "nvrtcCreateProgram failed";
     return false;
   }
@@ -134,7 +137,7 @@ struct DiagPlace {
   std::vector<int> tq, tbit;  // ... on thread bits, tile bits
   std::vector<int> gq;        // ... outside the tile
 };
-DiagPlace diag_place(const DevStageF& st, const DevOp& op, int rb) {
+DiagPlace diag_place(const uint32_t* dep, const DevOp& op, int rb) {
   DiagPlace d;
   for (int i = 0; i < op.nd; ++i) {
     if (op.dbit[i] < 0) {
@@ -143,7 +146,7 @@ DiagPlace diag_place(const DevStageF& st, const DevOp& op, int rb) {
     }
     int j = -1;
     for (int b = 0; b < rb; ++b)
-      if (st.dep[1 << b] == (1u << op.dbit[i])) j = b;
+      if (dep[1 << b] == (1u << op.dbit[i])) j = b;
     if (j == 0) {
       d.lane = i;
     } else if (j > 0) {
@@ -180,7 +183,7 @@ void emit_diag_index(std::ostringstream& os, const DiagPlace& d) {
   os << ";\n";
 }
 void emit_diag(std::ostringstream& os, const DevStageF& st, const DevOp& op, const char* cx, bool adj, int rb) {
-  const DiagPlace d = diag_place(st, op, rb);
+  const DiagPlace d = diag_place(st.dep, op, rb);
   const int np = 1 << (rb - 1), cls = diag_class(op.code);
   if (cls == kDiagTable) {
     emit_diag_index(os, d);
@@ -240,7 +243,7 @@ void emit_diag(std::ostringstream& os, const DevStageF& st, const DevOp& op, con
 // The bins of conj(lam) psi over the op's (at most two) qubits: sums per
 // register pattern first, then one placement into the thread's bin.
 void emit_accd(std::ostringstream& os, const DevStageF& st, const DevOp& op, int rb) {
-  const DiagPlace d = diag_place(st, op, rb);
+  const DiagPlace d = diag_place(st.dep, op, rb);
   const int np = 1 << (rb - 1);
   emit_diag_index(os, d);
   for (int p = 0; p < (1 << d.rq.size()); ++p) {
@@ -257,6 +260,23 @@ void emit_accd(std::ostringstream& os, const DevStageF& st, const DevOp& op, int
          << "        bin_add(s8, bi | " << (k | 1 << d.lane) << "u, hi(re) - hi(rn), hi(im));\n";
     os << "      }\n";
   }
+}
+
+// A diagonal table in the classic layout: register bit 0 is the "lane" place,
+// the others the pair bits.
+void emit_diag64(std::ostringstream& os, const DevStage& st, const DevOp& op, bool adj) {
+  const DiagPlace d = diag_place(st.dep, op, kRegBits);
+  emit_diag_index(os, d);
+  for (int p = 0; p < (1 << d.rq.size()); ++p)
+    for (int l = 0; l < (d.lane < 0 ? 1 : 2); ++l) {
+      os << "      { const double2 d = c[bi | " << (diag_pattern_index(d, p) | (d.lane < 0 ? 0 : l << d.lane)) << "u];\n";
+      for (int m : diag_pairs(d, p, 8))
+        for (int j = 2 * m + l; j < 2 * m + 2; j += d.lane < 0 ? 1 : 2) {
+          os << "        v[" << j << "] = tmul(d, v[" << j << "]);\n";
+          if (adj) os << "        w[" << j << "] = tmul(d, w[" << j << "]);\n";
+        }
+      os << "      }\n";
+    }
 }
 
 // The code of one op of a stage (o = its index in the pass's op array; cx =
@@ -453,6 +473,77 @@ std::string jit_pass_source(int M, bool adj, const DevStageF* st, int nst, const
   return os.str();
 }
 
+// Resident CTAs per SM of the compiled FP64 passes.  Forward: four 128-thread
+// CTAs (128 registers); reverse: VQC_JIT_MINB_ADJ64, default two (255 registers).
+int jit_min_blocks64(bool adj) { return adj ? env_int("VQC_JIT_MINB_ADJ64", 2) : env_int("VQC_JIT_MINB_FWD64", 4); }
+
+// An FP64 pass written out: the classic plan's stages and ops with the same
+// device functions as the interpreted body (tile_ops.cuh), so both give the
+// same bits.  Interpreting costs 3.4 instructions for every FP64 one on a
+// reverse pass (each op variant leaves the amplitudes in other registers, and
+// every switch moves all of them back), and the FP64 pipe idles at 25 %.
+std::string jit_pass_source64(int M, bool adj, const DevStage* st, int nst, const DevOp* ops, int npool) {
+  if (npool > kJitMaxCoef / 2) return std::string();  // beyond the kernel-parameter space: interpreted
+  std::ostringstream os;
+  os << "#include \"tile_ops.cuh\"\nusing namespace vqc;\n"
+     << "struct Coef { double2 c[" << std::max(npool, 1) << "]; };\n"
+     << "extern \"C\" __global__ void __launch_bounds__(" << (1 << (M - kRegBits)) << ", " << jit_min_blocks64(adj)
+     << ")\nvqc_pass64(const __grid_constant__ TileItem it, const __grid_constant__ Coef coef) {\n"
+     << "  constexpr bool ADJ = " << (adj ? "true" : "false") << ";\n"
+     << "  extern __shared__ __align__(16) unsigned char smem[];\n  __shared__ uint64_t s_tile[2];\n"
+     << "  TileRun<double, ADJ> x;\n  tile_begin<double, ADJ>(x, it, smem, s_tile, false);\n"
+     << "  double2 v[16], w[16];\n"
+     << "  for (int64_t tile = blockIdx.x; tile < it.p.ntiles; tile += it.ncta) {\n";
+  for (int s = 0; s < nst; ++s) {
+    os << "  {\n    const DevStage* S = x.stages + " << s << ";\n    constexpr uint32_t swm[16] = {";
+    for (int j = 0; j < 16; ++j) os << (j ? ", " : "") << st[s].swm[j] << "u";
+    os << "};\n    constexpr int64_t gdep[16] = {";
+    for (int j = 0; j < 16; ++j) os << (j ? ", " : "") << st[s].gdep[j] << "ll";
+    os << "};\n    tile_load<double, ADJ>(x, S, " << (s == 0 ? "true" : "false") << ", v, w, swm, gdep);\n"
+       << "    const uint32_t tthr = S->thr[0][x.tlo] | S->thr[1][x.thi];\n    (void)tthr;\n";
+    for (int o = st[s].op_begin; o < st[s].op_end; ++o) {
+      const DevOp& op = ops[o];
+      const int code = op.code, sel = (code >> kSelShift) & 127;
+      const bool acc = code & kCodeAcc;
+      const char* mk = sel & 4 ? "true" : "false";
+      const uint32_t rm = (uint32_t)op.rmask;
+      os << "    { const DevOp* op = x.ops + " << o << ";\n      (void)op;\n      const double2* c = coef.c + " << op.mat
+         << ";\n";
+      if (code & kCodeGCtl) os << "      if ((x.base & op->gmask) == op->gval) {\n";
+      os << "      const bool run = " << (code & kCodeCtl ? "(tthr & op->cmask) == op->cval" : "true")
+         << ";\n      if (run) {\n";
+      if (sel < kSelU2)
+        os << "        op_u1<" << (sel & 3) << ", " << mk << ", " << (sel >> 3) << ", ADJ>(v, w, c, " << rm << "u);\n";
+      else if (sel < kSelPhase)
+        os << "        op_u2<" << ((sel - kSelU2) >> 2) << ", " << ((sel - kSelU2) & 3) << ", ADJ>(v, w, c, " << rm
+           << "u);\n";
+      else if (sel == kSelPhase)
+        os << "        op_phase<ADJ>(v, w, c, " << rm << "u);\n";
+      else if (sel == kSelFlip)
+        os << "        op_flip<ADJ>(v, w, " << rm << "u);\n";
+      else if (sel == kSelDiag)
+        emit_diag64(os, st[s], op, adj);
+      os << "      }\n";
+      if (acc) {
+        const int kind = acc_kind_of(code);
+        os << "      double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};\n";
+        if (sel == kSelAccD)
+          os << "      op_accd<double>(v, w, op, tthr, S->dep, x.base, a);\n";
+        else
+          os << "      if (run) op_acc<" << (sel & 3) << ", " << mk << ", " << kind << ", double>(v, w, " << rm
+             << "u, a);\n";
+        os << "      flush_acc<" << (kind & kAccAH ? 4 : 8) << ">(a, tile_slot(x, op->slot));\n";
+      }
+      if (code & kCodeGCtl) os << "      }\n";
+      os << "    }\n";
+    }
+    os << "    tile_store<double, ADJ>(x, S, " << (s == nst - 1 ? "true" : "false") << ", v, w, swm, gdep, "
+       << (st[s].cta ? "true" : "false") << ");\n  }\n";
+  }
+  os << "    tile_advance(x);\n  }\n  tile_end(x, it);\n}\n";
+  return os.str();
+}
+
 // Kernels for `srcs` (nullptr where unavailable): cached ones at once, the
 // rest compiled in parallel, then loaded.
 namespace {
@@ -558,6 +649,150 @@ std::set<std::pair<uint64_t, uint64_t>>& inflight() {
   return s;
 }
 
+// What an op contributes to its pass's source.
+static void hash_ops(Hash128& h, const DevOp* ops, int begin, int end) {
+  h.val(begin);
+  h.val(end);
+  for (int o = begin; o < end; ++o) {
+    const DevOp& op = ops[o];
+    h.val(op.code);
+    h.val(op.mat);
+    h.val(op.rmask);
+    const int type = op.code & 15;
+    if (type == kOpDiag || type == kOpAccD) {  // (their places are written into the source)
+      h.val(op.nd);
+      h.add(op.dbit, sizeof(op.dbit));
+    }
+  }
+}
+
+// FP64 passes compile in the background: the first call with a structure runs
+// the interpreted kernels and queues the compile, the next call with it takes
+// the compiled kernel (waiting for it if it is not done yet), so a circuit that
+// runs once never waits.  Both kernels give the same bits.
+namespace {
+struct Job64 {
+  std::string src;
+  std::vector<char> cubin;
+  std::string log;
+  int state = 0;  // 0 queued or compiling, 1 done, 2 failed
+  uint64_t call = 0;
+};
+struct Background {
+  std::mutex mu;
+  std::condition_variable work, done;
+  std::deque<std::shared_ptr<Job64>> queue;
+  std::map<std::pair<uint64_t, uint64_t>, std::shared_ptr<Job64>> jobs;
+  std::vector<std::thread> threads;
+  bool stop = false;
+  void run() {
+    std::unique_lock<std::mutex> lk(mu);
+    while (true) {
+      work.wait(lk, [&] { return stop || !queue.empty(); });
+      if (stop) return;
+      auto j = queue.front();
+      queue.pop_front();
+      lk.unlock();
+      const bool ok = compile_one(j->src, j->cubin, j->log);
+      lk.lock();
+      j->state = ok ? 1 : 2;
+      j->src.clear();
+      done.notify_all();
+    }
+  }
+  void push(std::shared_ptr<Job64> j) {  // mu held
+    const size_t most = std::max(1u, std::thread::hardware_concurrency());
+    queue.push_back(j);
+    if (threads.size() < std::min(most, (size_t)64) && threads.size() < jobs.size()) threads.emplace_back([this] { run(); });
+    work.notify_one();
+  }
+  ~Background() {
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      stop = true;
+      work.notify_all();
+    }
+    for (auto& t : threads) t.join();  // (a compile in progress ends first)
+  }
+};
+Background& background() {
+  static Background b;
+  return b;
+}
+}  // namespace
+
+int jit_pass_kernels64(int M, bool adj, const std::vector<JitPassRef64>& refs, std::vector<const void*>& out,
+                       uint64_t call, bool wait) {
+  out.assign(refs.size(), nullptr);
+  if (!jit_available()) return VQC_OK;
+  const int flags[4] = {64, M, adj ? 1 : 0, jit_min_blocks64(adj)};
+  std::vector<std::pair<uint64_t, uint64_t>> keys(refs.size());
+  std::vector<std::shared_ptr<Job64>> jobs(refs.size());
+  Background& bg = background();
+  {
+    std::lock_guard<std::mutex> lk(bg.mu);
+    for (size_t i = 0; i < refs.size(); ++i) {
+      const JitPassRef64& r = refs[i];
+      if (!r.stages) continue;
+      Hash128 h;
+      h.add(flags, sizeof(flags));
+      h.val(r.nstages);
+      h.val(r.npool);
+      for (int s = 0; s < r.nstages; ++s) {
+        const DevStage& st = r.stages[s];
+        h.add(st.swm, sizeof(st.swm));
+        h.add(st.gdep, sizeof(st.gdep));
+        h.val(st.cta);
+        hash_ops(h, r.ops, st.op_begin, st.op_end);
+      }
+      keys[i] = {h.a, h.b};
+      auto it = bg.jobs.find(keys[i]);
+      if (it != bg.jobs.end()) {
+        jobs[i] = it->second;
+        continue;
+      }
+      auto j = std::make_shared<Job64>();
+      j->src = jit_pass_source64(M, adj, r.stages, r.nstages, r.ops, r.npool);
+      j->call = call;
+      jobs[i] = bg.jobs[keys[i]] = j;
+      if (j->src.empty())
+        j->state = 2;
+      else
+        bg.push(j);
+    }
+  }
+  long long compiled = 0;
+  for (size_t i = 0; i < refs.size(); ++i) {
+    if (!jobs[i] || (jobs[i]->call == call && !wait)) continue;
+    Job64& j = *jobs[i];
+    {
+      std::unique_lock<std::mutex> lk(bg.mu);
+      bg.done.wait(lk, [&] { return j.state != 0; });
+    }
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = hcache().find(keys[i]);
+    if (it != hcache().end()) {
+      out[i] = it->second;
+      continue;
+    }
+    cudaLibrary_t lib = nullptr;
+    cudaKernel_t k = nullptr;
+    const void* kernel = nullptr;
+    if (j.state == 1 &&
+        cudaLibraryLoadData(&lib, j.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) == cudaSuccess &&
+        cudaLibraryGetKernel(&k, lib, "vqc_pass64") == cudaSuccess)
+      kernel = (const void*)k;
+    else
+      cudaGetLastError();  // (the interpreted kernel runs the pass)
+    if (env_int("VQC_JIT_VERBOSE", 0)) fprintf(stderr, "vqc jit: %s\n", j.log.c_str());
+    std::vector<char>().swap(j.cubin);
+    out[i] = hcache()[keys[i]] = kernel;
+    ++compiled;
+  }
+  if (compiled) prof_note("jit_compiled_passes", compiled);
+  return VQC_OK;
+}
+
 int jit_pass_kernels(int M, bool adj, const std::vector<JitPassRef>& refs, std::vector<const void*>& out, bool batch,
                      bool compile, int rb) {
   out.assign(refs.size(), nullptr);
@@ -580,21 +815,7 @@ int jit_pass_kernels(int M, bool adj, const std::vector<JitPassRef>& refs, std::
         const DevStageF& st = r.stages[s];
         h.add(st.swm, sizeof(st.swm));
         h.add(st.gdep, sizeof(st.gdep));
-        h.val(st.op_begin);
-        h.val(st.op_end);
-        for (int o = st.op_begin; o < st.op_end; ++o) {
-          const DevOp& op = r.ops[o];
-          h.val(op.code);
-          h.val(op.mat);
-          const int type = op.code & 15;
-          if (type == kOpDiag || type == kOpAccD) {  // (their places and entry are written into the source)
-            h.val(op.nd);
-            h.add(op.dbit, sizeof(op.dbit));
-            if (diag_class(op.code) != kDiagTable) h.val(op.rmask);
-          } else if (type == kOpU2 || ((op.code >> 16) & 7) == 7) {
-            h.val(op.rmask);
-          }
-        }
+        hash_ops(h, r.ops, st.op_begin, st.op_end);
       }
       keys[i] = {h.a, h.b};
       auto it = hcache().find(keys[i]);

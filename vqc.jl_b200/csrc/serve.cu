@@ -285,6 +285,12 @@ static void fail_all(vqc_server_s* s, const std::string& why) {
     }                                                                  \
   } while (0)
 
+static DevPass pass_of(const SerialPlan& sp, const PassLoc& l) {
+  DevPass p;
+  std::memcpy(&p, sp.buf.data() + l.pass, sizeof(p));
+  return p;
+}
+
 static void worker_main(vqc_server_s* s) {
   if (cudaSetDevice(s->device) != cudaSuccess) {
     fail_all(s, "cudaSetDevice failed in the serving worker");
@@ -391,7 +397,7 @@ static void worker_main(vqc_server_s* s) {
         Group& g = groups[std::make_tuple(r->plan.M, 0, k)];
         g.items.push_back(TileItem{r->psi, nullptr, (const DevPass*)(img + l.pass), (const void*)(img + l.stages),
                                    (const DevOp*)(img + l.ops), img + r->plan.fwd.pool_off + l.pool_begin * amp,
-                                   nullptr, l.ntiles, r->fwd_cap, 0});
+                                   nullptr, l.ntiles, r->fwd_cap, r->plan.M, pass_of(r->plan.fwd, l)});
         g.reqs.push_back(r);
         g.locs.push_back(&l);
       } else if (r->step == F) {
@@ -407,7 +413,7 @@ static void worker_main(vqc_server_s* s) {
         Group& g = groups[std::make_tuple(r->plan.M, 1, k)];
         g.items.push_back(TileItem{r->psi, r->lam, (const DevPass*)(ai + l.pass), (const void*)(ai + l.stages),
                                    (const DevOp*)(ai + l.ops), ai + r->plan.adj.pool_off + l.pool_begin * amp,
-                                   r->partials, l.ntiles, r->adj_cap, 0});
+                                   r->partials, l.ntiles, r->adj_cap, r->plan.M, pass_of(r->plan.adj, l)});
         g.reqs.push_back(r);
         g.locs.push_back(&l);
         if (l.nslots > 0)

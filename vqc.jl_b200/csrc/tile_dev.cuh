@@ -8,6 +8,7 @@ typedef unsigned long long uint64_t;
 typedef long long int64_t;
 typedef unsigned int uint32_t;
 typedef int int32_t;
+typedef unsigned short uint16_t;
 #else
 #include <cstdint>
 #endif
@@ -23,7 +24,7 @@ namespace vqc {
 constexpr int kRegBits = 4;  // 16 amplitudes per thread
 constexpr int kMaxSlots = 64;
 constexpr int kMaxOpsPerPass = 192;  // bounds the pass's descriptors staged in shared memory
-enum { kOpU1 = 1, kOpU2 = 2, kOpDiag = 3, kOpAccD = 4 };
+enum { kOpU1 = 1, kOpU2 = 2, kOpDiag = 3, kOpAccD = 4, kOpPhase = 5 };
 
 struct DevPass {
   uint64_t nontile_mask;  // global bits enumerated by the tile counter
@@ -35,12 +36,19 @@ struct DevPass {
   int32_t pad;
 };
 
+// A stage of the classic tile body.  Per-thread quantities are split into two
+// tables indexed by the thread index's low and high nibble (thread bits are at
+// most 8), so no thread deposits bits at run time.
 struct alignas(16) DevStage {
-  uint32_t dep[16];    // tile index of register slot j (OR with the thread part)
-  int64_t gdep[16];    // global offset of register slot j
-  uint64_t gthr_mask;  // global qubits of the thread's tile bits
-  uint32_t thr_mask;   // tile bits held by the thread index, ascending
-  int32_t op_begin, op_end, pad;
+  int64_t gdep[16];     // global amplitude offset of register amplitude j
+  int64_t gthr[2][16];  // global offset of the thread's tile bits: [0][tid & 15] + [1][tid >> 4]
+  uint32_t thr[2][16];  // tile index of the thread's bits: [0][tid & 15] | [1][tid >> 4]
+  uint32_t swt[2][16];  // swizzled tile index of the thread's bits: [0][..] ^ [1][..]
+  uint32_t swm[16];     // swizzled tile index of register amplitude j
+  uint32_t dep[16];     // tile index of register amplitude j
+  int32_t op_begin, op_end;
+  int32_t cta;          // 0: the next stage keeps the warp index on the same tile bits (a warp barrier ends this one)
+  int32_t pad;
 };
 
 // A stage of the FP32 (packed) tile body: tile bit 0 is always a register
@@ -61,7 +69,7 @@ struct alignas(16) DevStageF {
 
 // code: bits 0-3 op type, 4-5 r0, 6-7 r1, 8 tile-bit controls, 9 non-tile
 // controls, 10 accumulate, 20-21 the third bits of r0 / r1.  The first 16 bytes are read as one vector load.
-// In the FP32 body, r0/r1 are j-bits (0 = lane bit, 1..3 or 1..4 = free
+// In the packed FP32 body, r0/r1 are j-bits (0 = lane bit, 1..3 or 1..4 = free
 // register bits), cmask/cval hold only the controls on thread bits, and the
 // controls on register bits are bits 16-18 (0: none, 1..5: one control on
 // j-bit value-1 at |1>, 7: the amplitudes enabled in rmask).
@@ -74,8 +82,21 @@ struct alignas(16) DevOp {
   int32_t nd;      // diagonal ops: number of qubits
   int32_t dbit[5];  // tile bit of diagonal qubit i, or -1
   int32_t dglob[5]; // global qubit of diagonal qubit i when not a tile bit
-  int32_t rmask;    // FP32 body: register amplitudes (pair representatives) the controls enable
+  int32_t rmask;    // register amplitudes (pair representatives) the controls enable
+  // classic body: the thread's amplitudes the op acts on, as swizzled tile
+  // indices: first ^ (any combination of the op_free(code) entries of step),
+  // with the target bits at 0; target: what flips a target bit
+  uint16_t first, step[3], target[2];
 };
+// The classic body's op variant (bits 24-30 of the code): one-qubit ops kSelU1
+// + (r0 | masked << 2 | form << 3), masked = a register control in rmask;
+// two-qubit ops kSelU2 + (r0 * 4 + r1); a phase on the amplitudes the controls
+// enable (a diagonal gate with one entry that is not 1), a flip of sign (that
+// entry is -1); a full diagonal table; its bins.  Bits 16-18: free register
+// bits (neither target nor control).
+constexpr int kSelShift = 24;
+__host__ __device__ constexpr int op_free(int code) { return (code >> 16) & 7; }
+enum { kSelU1 = 0, kSelU2 = 64, kSelPhase = 96, kSelFlip = 97, kSelDiag = 98, kSelAccD = 99 };
 constexpr int kCodeCtl = 1 << 8, kCodeGCtl = 1 << 9, kCodeAcc = 1 << 10;
 // r0 / r1 as 3-bit j-bits (the wide FP32 body has j-bits 0..4): bits 4-5 and
 // 6-7 hold the low two bits, bits 20 and 21 the third.
@@ -119,7 +140,8 @@ struct TileItem {
   double* partials;  // [ncta][nslots][8]
   int64_t ntiles;
   int ncta;
-  int pad;
+  int M;      // tile bits
+  DevPass p;  // *pass, by value: one dependent load fewer before the descriptors
 };
 
 // Shared-memory bytes of the FP32 tile(s) of one pass.

@@ -1,15 +1,5 @@
-// Tile kernels: FP32 classic body and the serving batch kernel, forward passes.
+// Tile kernels: the classic body, FP32, forward passes.
 #include "tile_kernels_impl.cuh"
 
-VQC_INST_TILE(float, 9, false, true, false)
-VQC_INST_TILE(float, 9, false, false, false)
-VQC_INST_TILE(float, 10, false, true, false)
-VQC_INST_TILE(float, 10, false, false, false)
-VQC_INST_TILE(float, 11, false, true, false)
-VQC_INST_TILE(float, 11, false, false, false)
-VQC_INST_TILE(float, 12, false, true, false)
-VQC_INST_TILE(float, 12, false, false, false)
-VQC_INST_BATCH(float, 9, false)
-VQC_INST_BATCH(float, 10, false)
-VQC_INST_BATCH(float, 11, false)
-VQC_INST_BATCH(float, 12, false)
+template __global__ void vqc::k_tile<float, false>(const __grid_constant__ vqc::TileItem);
+template __global__ void vqc::k_tile_batch<float, false>(const vqc::TileItem*);

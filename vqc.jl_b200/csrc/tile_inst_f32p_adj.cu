@@ -1,11 +1,7 @@
-// Tile kernels: FP32 packed body (interpreted form of the compiled passes), reverse sweep.
+// Tile kernels: the FP32 packed body (interpreted form of the compiled passes), reverse sweep.
 #include "tile_kernels_impl.cuh"
 
-VQC_INST_TILE(float, 9, true, true, true)
-VQC_INST_TILE(float, 9, true, false, true)
-VQC_INST_TILE(float, 10, true, true, true)
-VQC_INST_TILE(float, 10, true, false, true)
-VQC_INST_TILE(float, 11, true, true, true)
-VQC_INST_TILE(float, 11, true, false, true)
-VQC_INST_TILE(float, 12, true, true, true)
-VQC_INST_TILE(float, 12, true, false, true)
+template __global__ void vqc::k_tile_packed<9, true>(const __grid_constant__ vqc::TileItem);
+template __global__ void vqc::k_tile_packed<10, true>(const __grid_constant__ vqc::TileItem);
+template __global__ void vqc::k_tile_packed<11, true>(const __grid_constant__ vqc::TileItem);
+template __global__ void vqc::k_tile_packed<12, true>(const __grid_constant__ vqc::TileItem);

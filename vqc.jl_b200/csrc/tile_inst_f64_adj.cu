@@ -1,12 +1,5 @@
-// Tile kernels: FP64 body and the serving batch kernel, reverse sweep.
+// Tile kernels: the classic body, FP64, reverse sweep.
 #include "tile_kernels_impl.cuh"
 
-VQC_INST_TILE(double, 9, true, true, false)
-VQC_INST_TILE(double, 9, true, false, false)
-VQC_INST_TILE(double, 10, true, true, false)
-VQC_INST_TILE(double, 10, true, false, false)
-VQC_INST_TILE(double, 11, true, true, false)
-VQC_INST_TILE(double, 11, true, false, false)
-VQC_INST_BATCH(double, 9, true)
-VQC_INST_BATCH(double, 10, true)
-VQC_INST_BATCH(double, 11, true)
+template __global__ void vqc::k_tile<double, true>(const __grid_constant__ vqc::TileItem);
+template __global__ void vqc::k_tile_batch<double, true>(const vqc::TileItem*);

@@ -1,12 +1,5 @@
-// Tile kernels: FP64 body and the serving batch kernel, forward passes.
+// Tile kernels: the classic body, FP64, forward passes.
 #include "tile_kernels_impl.cuh"
 
-VQC_INST_TILE(double, 9, false, true, false)
-VQC_INST_TILE(double, 9, false, false, false)
-VQC_INST_TILE(double, 10, false, true, false)
-VQC_INST_TILE(double, 10, false, false, false)
-VQC_INST_TILE(double, 11, false, true, false)
-VQC_INST_TILE(double, 11, false, false, false)
-VQC_INST_BATCH(double, 9, false)
-VQC_INST_BATCH(double, 10, false)
-VQC_INST_BATCH(double, 11, false)
+template __global__ void vqc::k_tile<double, false>(const __grid_constant__ vqc::TileItem);
+template __global__ void vqc::k_tile_batch<double, false>(const vqc::TileItem*);

@@ -7,14 +7,15 @@
 
 namespace vqc {
 
-// One pass of one state: the tiles of the pass strided over the grid.  GEN =
-// false: every op is a one-qubit op; PACKED: the FP32 packed body
-// (tile_f32.cuh) on a plan laid out for it.
-template <class R, int M, bool ADJ, bool GEN, bool PACKED>
-__global__ void k_tile(cplx<R>* psi, cplx<R>* lam, const DevPass* pass, const void* stages, const DevOp* ops,
-                       const cplx<R>* pool, double* partials);
+// One pass of one state: the tiles of the pass strided over the grid.
+template <class R, bool ADJ>
+__global__ void k_tile(const __grid_constant__ TileItem item);
 // One pass each of many states (the serving loop): item blockIdx.y.
-template <class R, int M, bool ADJ>
+template <class R, bool ADJ>
 __global__ void k_tile_batch(const TileItem* __restrict__ items);
+// One pass of one FP32 state on the packed plan, interpreted (the fallback of
+// a compiled pass).
+template <int M, bool ADJ>
+__global__ void k_tile_packed(const __grid_constant__ TileItem item);
 
 }  // namespace vqc

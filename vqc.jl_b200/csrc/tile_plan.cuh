@@ -10,14 +10,18 @@
 
 namespace vqc {
 
-// Shared-memory bytes of one pass: tiles, accumulation slots, and the pass's
-// own stage / op / matrix descriptors (read by every thread for every op, so
-// they are staged once per CTA instead of being fetched through L1/L2).
-template <class R, int M, bool ADJ>
-__host__ __device__ constexpr size_t tile_bytes() {
-  return (size_t)(ADJ ? 2 : 1) * (size_t(1) << M) * sizeof(cplx<R>);
-}
-
+// XOR swizzle of a tile index in shared memory (classic body), linear over
+// XOR, so an address is the thread's part ^ the register amplitude's part.
+template <class R>
+struct Swz;
+template <>
+struct Swz<float> {  // 8-byte amplitudes: half-warps must hit 16 distinct 8-byte bank pairs
+  __host__ __device__ static __forceinline__ uint32_t f(uint32_t t) { return t ^ ((t >> 4) & 15u); }
+};
+template <>
+struct Swz<double> {  // 16-byte amplitudes: quarter-warps must hit 8 distinct 16-byte bank quads
+  __host__ __device__ static __forceinline__ uint32_t f(uint32_t t) { return t ^ (((t >> 3) ^ (t >> 6)) & 7u); }
+};
 
 struct PGrad {
   int param;             // caller's parameter index
@@ -38,7 +42,6 @@ struct FOp {
 
 struct PassShape {
   int nslots = 0, nstages = 0, nops = 0, npool = 0;
-  bool general = true;  // false: every op of the pass is a one-qubit op
   bool packed = false;  // FP32 packed layout (DevStageF), for the compiled pass kernels
 };
 
@@ -158,6 +161,21 @@ struct JitPassRef {
 // kWideRegBits for wide forward passes).
 int jit_pass_kernels(int M, bool adj, const std::vector<JitPassRef>& refs, std::vector<const void*>& out,
                      bool batch = false, bool compile = true, int rb = kRegBits);
+
+// The same for FP64 passes (the classic plan).  `call` names the user's call
+// the passes belong to: a structure first seen in it runs interpreted while it
+// compiles in the background; one seen in an earlier call is waited for.
+// wait: compile at once.
+struct JitPassRef64 {
+  const DevStage* stages = nullptr;
+  int nstages = 0;
+  const DevOp* ops = nullptr;
+  int npool = 0;
+};
+int jit_min_blocks64(bool adj);
+std::string jit_pass_source64(int M, bool adj, const DevStage* stages, int nstages, const DevOp* ops, int npool);
+int jit_pass_kernels64(int M, bool adj, const std::vector<JitPassRef64>& refs, std::vector<const void*>& out,
+                       uint64_t call, bool wait);
 
 // compiled: an FP32 packed plan with compiled batch kernels (fwd_k / adj_k)
 // when every pass has one already, else the classic plan for the generic

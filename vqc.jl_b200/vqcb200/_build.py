@@ -47,7 +47,8 @@ def _compile(src, extra, build_dir=BUILD):
     return obj, r.stderr
 
 
-JIT_HEADERS = [("kJitTileDev", "tile_dev.cuh"), ("kJitTileF32", "tile_f32.cuh")]
+JIT_HEADERS = [("kJitTileDev", "tile_dev.cuh"), ("kJitTileF32", "tile_f32.cuh"), ("kJitCplx", "cplx.cuh"),
+               ("kJitTileOps", "tile_ops.cuh")]
 
 
 def write_jit_sources(build_dir=BUILD):
