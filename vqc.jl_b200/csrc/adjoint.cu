@@ -23,7 +23,7 @@ namespace vqc {
 
 int pauli_run(vqc_state h, const void* bra, const void* ket, void* out, const vqc_pauli* terms, int nterms,
               bool write, bool acc, bool hermitian_part, double* result, bool* deferred = nullptr);
-int expect_dense_device(vqc_state h, const void* bra, const void* ket, int k, const int* sp, const std::vector<cd>& M,
+int expect_dense_device(vqc_state h, const void* bra, const void* ket, int k, const int* sp, const Mat& M,
                         double* res);
 int apply_circuit_raw(vqc_state h, const vqc_gate* gates, int ngates, const double* mats, bool dm, int fuse);
 
@@ -190,7 +190,7 @@ int prepare_reverse(int nq, const vqc_gate* gates, int ngates, const double* mat
     const int d = 1 << gs.k;
     for (ParamInfo& pi : per_gate[i]) {
       int sp[5];
-      std::vector<cd> dU;
+      Mat dU;
       const vqc_param& pr = params[pi.index];
       if (pr.kind != VQC_PARAM_DERIVATIVE && pr.kind != VQC_PARAM_GENERATOR)
         return fail(VQC_ERR_ARG, "unknown parameter kind");

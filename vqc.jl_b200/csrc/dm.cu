@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kRedThreads)
 }
 
 template <int K>
-static int trace_prod_k(vqc_state a, vqc_state b, int dag_a, int dag_b, const int* sp, const std::vector<cd>& M,
+static int trace_prod_k(vqc_state a, vqc_state b, int dag_a, int dag_b, const int* sp, const Mat& M,
                         double* out) {
   TraceProdArgs<K> g;
   for (int i = 0; i < (1 << K) * (1 << K); ++i) g.M[i] = make_double2(M[i].real(), M[i].imag());
@@ -268,7 +268,7 @@ int vqc_dm_trace_prod(vqc_state a, int dag_a, vqc_state b, int dag_b, int k, con
   if (k < 1 || k > 5) return fail(VQC_ERR_UNSUPPORTED, "only implement 5-qubit gates and less currently.");
   if (k > b->n_dm) return fail(VQC_ERR_ARG, "operator wider than the register");
   int sp[5];
-  std::vector<cd> M;
+  Mat M;
   if ((rc = order_matrix(b->n_dm, k, pos, mat, sp, M))) return rc;
   std::lock_guard<std::mutex> lk(b->mu);
   std::unique_lock<std::mutex> la(a->mu, std::defer_lock);

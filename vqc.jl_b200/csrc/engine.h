@@ -3,6 +3,9 @@
 #pragma once
 
 #include <complex>
+#include <cstring>
+#include <initializer_list>
+#include <memory>
 #include <vector>
 
 #include "common.cuh"
@@ -10,6 +13,72 @@
 namespace vqc {
 
 using cd = std::complex<double>;
+
+// A small complex matrix: up to N entries in place, more on the heap.  Planning
+// a circuit makes several for every gate; with std::vector their allocations
+// were half of the host time of a gradient of a few hundred gates.
+template <int N>
+class SmallMat {
+ public:
+  SmallMat() {}
+  explicit SmallMat(size_t n, cd v = cd(0)) { assign(n, v); }
+  SmallMat(std::initializer_list<cd> l) { copy(l.begin(), l.size()); }
+  SmallMat(const SmallMat& o) { copy(o.data(), o.n_); }
+  SmallMat(SmallMat&& o) noexcept { take(o); }
+  template <int K>
+  SmallMat(const SmallMat<K>& o) { copy(o.data(), o.size()); }
+  SmallMat& operator=(const SmallMat& o) {
+    if (this != &o) copy(o.data(), o.n_);
+    return *this;
+  }
+  SmallMat& operator=(SmallMat&& o) noexcept {
+    if (this != &o) take(o);
+    return *this;
+  }
+  void assign(size_t n, cd v) {
+    reserve(n);
+    for (size_t i = 0; i < n; ++i) data()[i] = v;
+  }
+  size_t size() const { return n_; }
+  bool empty() const { return n_ == 0; }
+  cd* data() { return heap_ ? heap_.get() : reinterpret_cast<cd*>(in_); }
+  const cd* data() const { return heap_ ? heap_.get() : reinterpret_cast<const cd*>(in_); }
+  cd& operator[](size_t i) { return data()[i]; }
+  const cd& operator[](size_t i) const { return data()[i]; }
+  cd* begin() { return data(); }
+  cd* end() { return data() + n_; }
+  const cd* begin() const { return data(); }
+  const cd* end() const { return data() + n_; }
+
+ private:
+  void reserve(size_t n) {
+    if (n > cap_) {
+      heap_.reset(new cd[n]);
+      cap_ = n;
+    }
+    n_ = n;
+  }
+  void copy(const cd* p, size_t n) {
+    reserve(n);
+    if (n) std::memcpy((void*)data(), (const void*)p, n * sizeof(cd));
+  }
+  void take(SmallMat& o) {
+    if (!o.heap_) {
+      copy(o.data(), o.n_);
+      return;
+    }
+    heap_ = std::move(o.heap_);
+    cap_ = o.cap_;
+    n_ = o.n_;
+    o.cap_ = N;
+    o.n_ = 0;
+  }
+  size_t n_ = 0, cap_ = N;
+  std::unique_ptr<cd[]> heap_;
+  alignas(16) double in_[2 * N];  // (not initialised)
+};
+using Mat = SmallMat<16>;   // gates of up to two qubits in place
+using Mat2 = SmallMat<4>;   // 2x2
 
 // A gate reduced to the part of the state it changes.
 //
@@ -24,11 +93,11 @@ using cd = std::complex<double>;
 struct GateSpec {
   int k = 0;
   int sp[5] = {0, 0, 0, 0, 0};  // sorted positions
-  std::vector<cd> U;            // 2^k x 2^k, bit b <-> sp[b]
+  Mat U;                        // 2^k x 2^k, bit b <-> sp[b]
   int ns = 0;                   // |S|
   int S[32];                    // active indices, ascending
   int mode = 0;                 // kDense / kDiag / kMono on U[S][S]
-  std::vector<cd> US;           // ns x ns
+  Mat US;                       // ns x ns
   int mono_src[32];             // kMono: out_a = US[a][mono_src[a]] * in_{mono_src[a]}
 };
 constexpr int kDense = 0, kDiag = 1, kMono = 2;
@@ -37,13 +106,13 @@ constexpr int kDense = 0, kDiag = 1, kMono = 2;
 // finds its active subspace.  dagger: analyse U^dagger instead of U.
 int analyze_gate(int n, int k, const int* pos, const double* mat, bool dagger, GateSpec& g);
 // Sorted-order matrix of an arbitrary operator (no unitarity assumed).
-int order_matrix(int n, int k, const int* pos, const double* mat, int* sp, std::vector<cd>& M);
+int order_matrix(int n, int k, const int* pos, const double* mat, int* sp, Mat& M);
 
 // One circuit parameter in the reverse sweep: D = U^dagger dU/dtheta (or
 // G^dagger for generator-kind parameters), sorted order, 2^k x 2^k.
 struct ParamInfo {
   int index;  // position in the caller's params array
-  std::vector<cd> D;
+  Mat D;
 };
 
 int prepare_reverse(int nq, const vqc_gate* gates, int ngates, const double* mats, const vqc_param* params,

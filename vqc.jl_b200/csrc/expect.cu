@@ -1548,7 +1548,7 @@ __global__ void __launch_bounds__(256)
 }
 
 template <int MS>
-static void fill_dense(int nq, int k, const int* sp, const std::vector<cd>& M, DenseArgs<MS>& a) {
+static void fill_dense(int nq, int k, const int* sp, const Mat& M, DenseArgs<MS>& a) {
   a.ngroups = mask_of(k, sp, nq, a.mask);
   for (int j = k + 1; j < 6; ++j) a.mask[j] = 0;
   a.k = k;
@@ -1558,7 +1558,7 @@ static void fill_dense(int nq, int k, const int* sp, const std::vector<cd>& M, D
 
 template <int MS>
 static int expect_dense_ms(vqc_state h, const void* bra, const void* ket, int k, const int* sp,
-                           const std::vector<cd>& M, double* res) {
+                           const Mat& M, double* res) {
   DenseArgs<MS> a;
   fill_dense<MS>(h->nq, k, sp, M, a);
   const int grid = reduction_grid(h->device, a.ngroups);
@@ -1573,7 +1573,7 @@ static int expect_dense_ms(vqc_state h, const void* bra, const void* ket, int k,
 }
 
 // sum conj(bra) M ket over the key's groups into res[0..1] (device).
-int expect_dense_device(vqc_state h, const void* bra, const void* ket, int k, const int* sp, const std::vector<cd>& M,
+int expect_dense_device(vqc_state h, const void* bra, const void* ket, int k, const int* sp, const Mat& M,
                         double* res) {
   switch (k) {
     case 1: return expect_dense_ms<2>(h, bra, ket, k, sp, M, res);
@@ -1585,7 +1585,7 @@ int expect_dense_device(vqc_state h, const void* bra, const void* ket, int k, co
 }
 
 template <int MS>
-static int apply_dense_ms(vqc_state h, const void* ket, void* out, int k, const int* sp, const std::vector<cd>& M) {
+static int apply_dense_ms(vqc_state h, const void* ket, void* out, int k, const int* sp, const Mat& M) {
   DenseArgs<MS> a;
   fill_dense<MS>(h->nq, k, sp, M, a);
   const int grid = launch_grid(h->device, a.ngroups);
@@ -1687,7 +1687,7 @@ int vqc_expect_dense(vqc_state phi, vqc_state psi, int k, const int* pos, const 
     return fail(VQC_ERR_ARG, "expectation: states differ in size, dtype or device");
   std::lock_guard<std::mutex> lk(psi->mu);
   int sp[5];
-  std::vector<cd> M;
+  Mat M;
   if ((rc = order_matrix(psi->nq, k, pos, mat, sp, M))) return rc;
   if (phi && (rc = stream_after(psi, phi))) return rc;
   if ((rc = expect_dense_device(psi, phi ? phi->d : psi->d, psi->d, k, sp, M, psi->scr.result))) return rc;
@@ -1704,7 +1704,7 @@ int vqc_apply_dense_add(vqc_state psi, vqc_state out, int k, const int* pos, con
     return fail(VQC_ERR_ARG, "apply: output must be a distinct state of the same size, dtype and device");
   std::lock_guard<std::mutex> lk(psi->mu);
   int sp[5];
-  std::vector<cd> M;
+  Mat M;
   if ((rc = order_matrix(psi->nq, k, pos, mat, sp, M))) return rc;
   if ((rc = stream_after(psi, out))) return rc;
   switch (k) {

@@ -34,6 +34,7 @@
 #include <mutex>
 #include <set>
 #include <thread>
+#include <tuple>
 #include <type_traits>
 
 #include "engine.h"
@@ -83,7 +84,7 @@ static bool to_fop(const GateSpec& g, FOp& f) {
     f.kind = kOpDiag;
     f.nd = k;
     for (int b = 0; b < k; ++b) f.dq[b] = g.sp[b];
-    f.mat.resize(d);
+    f.mat.assign(d, cd(0));
     for (int j = 0; j < d; ++j) f.mat[j] = g.U[(size_t)j * d + j];
     return true;
   }
@@ -127,7 +128,7 @@ static bool to_fop(const GateSpec& g, FOp& f) {
 }
 
 // Restriction of a full sorted-order k-qubit matrix to the op's target subspace.
-static std::vector<cd> restrict_to(const GateSpec& g, const FOp& f, const std::vector<cd>& D) {
+static Mat2 restrict_to(const GateSpec& g, const FOp& f, const Mat& D) {
   const int k = g.k, d = 1 << k;
   int cval_bits = 0, tb[2], nt = 0;
   for (int b = 0; b < k; ++b) {
@@ -139,7 +140,7 @@ static std::vector<cd> restrict_to(const GateSpec& g, const FOp& f, const std::v
     }
   }
   const int dn = 1 << nt;
-  std::vector<cd> R((size_t)dn * dn);
+  Mat2 R((size_t)dn * dn);
   auto full = [&](int a) {
     int j = cval_bits;
     for (int i = 0; i < nt; ++i)
@@ -151,13 +152,16 @@ static std::vector<cd> restrict_to(const GateSpec& g, const FOp& f, const std::v
   return R;
 }
 
-static void mat2_mul(const std::vector<cd>& A, const std::vector<cd>& B, std::vector<cd>& C) {  // C = A B
-  C.assign(4, cd(0));
+template <class A, class B>
+static Mat2 mat2_mul(const A& a, const B& b) {
+  Mat2 c(4);
   for (int r = 0; r < 2; ++r)
-    for (int c = 0; c < 2; ++c) C[r * 2 + c] = A[r * 2] * B[c] + A[r * 2 + 1] * B[2 + c];
+    for (int k = 0; k < 2; ++k) c[r * 2 + k] = a[r * 2] * b[k] + a[r * 2 + 1] * b[2 + k];
+  return c;
 }
-static std::vector<cd> mat2_dag(const std::vector<cd>& A) {
-  return {std::conj(A[0]), std::conj(A[2]), std::conj(A[1]), std::conj(A[3])};
+template <class A>
+static Mat2 mat2_dag(const A& a) {
+  return {std::conj(a[0]), std::conj(a[2]), std::conj(a[1]), std::conj(a[3])};
 }
 
 struct PlanStage {
@@ -172,6 +176,11 @@ struct PlanPass {
   std::vector<PlanStage> stages;
   int nslots = 0;
 };
+
+static void tile_bits(const PlanPass& p, int (&tbit)[64]) {
+  for (int& b : tbit) b = -1;
+  for (int b = 0; b < (int)p.tile_q.size(); ++b) tbit[p.tile_q[b]] = b;
+}
 
 struct TileConfig {
   int M;      // tile bits
@@ -242,21 +251,16 @@ static void plan_passes(int n, const TileConfig& tc, bool adj, std::vector<PItem
           FOp& g = p.ops[prev];
           if (g.kind == kOpU1 && g.cmask == 0 && g.tq[0] == f.tq[0]) {
             // g applied first, then f: merged = f.mat * g.mat
-            std::vector<cd> merged;
-            mat2_mul(f.mat, g.mat, merged);
+            const Mat2 merged = mat2_mul(f.mat, g.mat);
             if (adj) {
               // g's gradients were taken at g's output side = f's input: move them
-              // to the block input (f is applied after g, so D -> F^dag D F)
-              const std::vector<cd> Fd = mat2_dag(f.mat);
-              for (PGrad& pg : g.grads) {
-                std::vector<cd> t1, t2;
-                // in the reverse sweep the op matrices are U^dagger: f.mat = U_f^dagger,
-                // the block input lies after f, and D_g moves by conjugation with f.mat^dagger
-                mat2_mul(pg.D, Fd, t1);
-                mat2_mul(f.mat, t1, t2);
-                pg.D = t2;
-              }
-              for (PGrad& pg : f.grads) g.grads.push_back(pg);
+              // to the block input (f is applied after g, so D -> F^dag D F); in
+              // the reverse sweep the op matrices are U^dagger: f.mat = U_f^dagger,
+              // the block input lies after f, and D_g moves by conjugation with
+              // f.mat^dagger
+              const Mat2 Fd = mat2_dag(f.mat);
+              for (PGrad& pg : g.grads) pg.D = mat2_mul(f.mat, mat2_mul(pg.D, Fd));
+              for (PGrad& pg : f.grads) g.grads.push_back(std::move(pg));
               if (f.acc && !g.acc) {
                 g.acc = true;
                 ++p.nslots;
@@ -268,9 +272,8 @@ static void plan_passes(int n, const TileConfig& tc, bool adj, std::vector<PItem
         }
       }
       if (adj && f.acc) ++p.nslots;
-      p.ops.push_back(f);
-      for (int q = 0; q < n; ++q)
-        if (qs >> q & 1) last_on[q] = (int)p.ops.size() - 1;
+      p.ops.push_back(std::move(f));
+      for (uint64_t m = qs; m; m &= m - 1) last_on[__builtin_ctzll(m)] = (int)p.ops.size() - 1;
     }
     // fill the tile with the lowest remaining qubits
     for (int q = 0; q < n && popc64(Q) < M; ++q) Q |= 1ull << q;
@@ -285,30 +288,21 @@ static void plan_passes(int n, const TileConfig& tc, bool adj, std::vector<PItem
 // FP32: 8-byte amplitudes, half-warps over Swz<float>.  Packed FP32: 16-byte
 // pairs, the lowest three thread bits (tile bits outside rs, ascending) must
 // fall in distinct classes of the pair swizzle, class = (tile bit - 1) mod 3.
-static bool rs_conflict_free(const std::vector<int>& rs, int M, int dtype, bool packed) {
-  if (packed) {
-    int seen = 0, k = 0;
-    for (int b = 1; b < M && k < 3; ++b) {
-      if (std::find(rs.begin(), rs.end(), b) != rs.end()) continue;
-      const int res = (b - 1) % 3;
-      if (seen >> res & 1) return false;
-      seen |= 1 << res;
-      ++k;
-    }
-    return true;
-  }
-  std::vector<int> lanes;
-  for (int b = 0; b < M && (int)lanes.size() < (dtype == VQC_C64 ? 4 : 3); ++b)
-    if (std::find(rs.begin(), rs.end(), b) == rs.end()) lanes.push_back(b);
-  int seen = 0;
-  for (int b : lanes) {
+static bool rs_conflict_free(uint32_t rs, int M, int dtype, bool packed) {
+  const int want = packed || dtype != VQC_C64 ? 3 : 4;
+  int seen = 0, k = 0;
+  for (int b = packed ? 1 : 0; b < M && k < want; ++b) {
+    if (rs >> b & 1) continue;
     int res;
-    if (dtype == VQC_C64)
+    if (packed)
+      res = (b - 1) % 3;
+    else if (dtype == VQC_C64)
       res = b < 4 ? b : (b < 8 ? b - 4 : -1);
     else
       res = b < 3 ? b : (b < 9 ? (b - 3) % 3 : -1);
     if (res < 0 || (seen >> res & 1)) return false;
     seen |= 1 << res;
+    ++k;
   }
   return true;
 }
@@ -319,18 +313,24 @@ static bool rs_conflict_free(const std::vector<int>& rs, int M, int dtype, bool 
 // stage's control bits (register controls are compile-time cases in the FP32
 // body), then a bank-conflict-free layout.
 static void plan_stages(PlanPass& p, int M, int dtype, bool packed, int rb = kRegBits) {
-  const bool lane0 = packed;
   p.stages.clear();
-  std::map<int, int> tbit;  // global qubit -> tile bit
-  for (int b = 0; b < (int)p.tile_q.size(); ++b) tbit[p.tile_q[b]] = b;
-  std::vector<int> pending(p.ops.size());
+  int tbit[64];  // global qubit -> tile bit, -1 outside the tile
+  tile_bits(p, tbit);
+  auto tile_mask_of = [&](uint64_t qubits) {
+    uint32_t t = 0;
+    for (uint64_t m = qubits; m; m &= m - 1) {
+      const int b = tbit[__builtin_ctzll(m)];
+      if (b >= 0) t |= 1u << b;
+    }
+    return t;
+  };
+  std::vector<int> pending(p.ops.size()), rest;
   for (size_t i = 0; i < pending.size(); ++i) pending[i] = (int)i;
   while (!pending.empty()) {
     PlanStage st;
     uint64_t blocked = 0;
-    std::vector<int> rest;
-    std::vector<int> rs;
-    if (lane0) rs.push_back(0);
+    uint32_t rs = packed ? 1u : 0u;
+    rest.clear();
     for (int oi : pending) {
       const FOp& f = p.ops[oi];
       if (f.qubits & blocked) {
@@ -338,13 +338,10 @@ static void plan_stages(PlanPass& p, int M, int dtype, bool packed, int rb = kRe
         rest.push_back(oi);
         continue;
       }
-      std::vector<int> need;
-      if (f.kind == kOpU1) need = {tbit[f.tq[0]]};
-      if (f.kind == kOpU2) need = {tbit[f.tq[0]], tbit[f.tq[1]]};
-      std::vector<int> u = rs;
-      for (int b : need)
-        if (std::find(u.begin(), u.end(), b) == u.end()) u.push_back(b);
-      if ((int)u.size() <= rb) {
+      uint32_t u = rs;
+      if (f.kind == kOpU1 || f.kind == kOpU2) u |= 1u << tbit[f.tq[0]];
+      if (f.kind == kOpU2) u |= 1u << tbit[f.tq[1]];
+      if (__builtin_popcount(u) <= rb) {
         rs = u;
         st.ops.push_back(oi);
       } else {
@@ -352,40 +349,35 @@ static void plan_stages(PlanPass& p, int M, int dtype, bool packed, int rb = kRe
         rest.push_back(oi);
       }
     }
-    // fill the register set to 4 bits: control bits of the stage's ops first
-    std::vector<int> cand;
-    for (int oi : st.ops) {
-      const FOp& f = p.ops[oi];
-      for (int q = 0; q < 64; ++q)
-        if ((f.cmask >> q & 1) && tbit.count(q)) {
-          const int b = tbit[q];
-          if (std::find(rs.begin(), rs.end(), b) == rs.end() && std::find(cand.begin(), cand.end(), b) == cand.end())
-            cand.push_back(b);
-        }
-    }
+    // fill the register set to rb bits: control bits of the stage's ops first
+    int cand[64], nc = 0;
+    uint32_t listed = rs;
+    for (int oi : st.ops)
+      for (uint32_t m = tile_mask_of(p.ops[oi].cmask); m; m &= m - 1) {
+        const int b = __builtin_ctz(m);
+        if (!(listed >> b & 1)) cand[nc++] = b;
+        listed |= 1u << b;
+      }
     for (int b = 0; b < M; ++b)
-      if (std::find(rs.begin(), rs.end(), b) == rs.end() && std::find(cand.begin(), cand.end(), b) == cand.end())
-        cand.push_back(b);
-    const int need_more = rb - (int)rs.size();
-    std::vector<int> best;
+      if (!(listed >> b & 1)) cand[nc++] = b;
+    const int need_more = rb - __builtin_popcount(rs);
+    nc = std::min(nc, 10);
+    uint32_t best = 0;
     bool found = false;
-    const int nc = std::min((int)cand.size(), 10);
     for (int mask = 0; mask < (1 << nc) && !found; ++mask) {
-      if (popc64((uint64_t)mask) != need_more) continue;
-      std::vector<int> t = rs;
-      for (int i = 0; i < nc; ++i)
-        if (mask >> i & 1) t.push_back(cand[i]);
-      std::sort(t.begin(), t.end());
-      if (best.empty()) best = t;
+      if (__builtin_popcount(mask) != need_more) continue;
+      uint32_t t = rs;
+      for (int m = mask; m; m &= m - 1) t |= 1u << cand[__builtin_ctz(m)];
+      if (!best) best = t;
       if (rs_conflict_free(t, M, dtype, packed)) {
         best = t;
         found = true;
       }
     }
     if (!found) prof_note("plan_stages_bank_conflicted", 1);
-    st.rs = best;
-    p.stages.push_back(st);
-    pending = rest;
+    for (uint32_t m = best; m; m &= m - 1) st.rs.push_back(__builtin_ctz(m));
+    p.stages.push_back(std::move(st));
+    pending.swap(rest);
   }
 }
 
@@ -441,14 +433,26 @@ static int allow_smem(int device, const void* k) {
   return VQC_OK;
 }
 
-// Resident CTAs of a tile kernel over the whole device.
+// Resident CTAs of a tile kernel over the whole device (the occupancy query
+// costs a microsecond or two, for every pass of every call: kept per kernel and
+// shared-memory size).
 static int kernel_grid(int device, const void* k, int nt, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, int, size_t>, int> known;
+  const auto key = std::make_tuple(device, k, nt, smem);
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find(key);
+    if (it != known.end()) return it->second;
+  }
   int per_sm = 0;
-  if (allow_smem(device, k) || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, smem) != cudaSuccess || per_sm < 1) {
+  if (allow_smem(device, k) ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, nt, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     per_sm = 1;
   }
-  return device_info(device).sms * per_sm;
+  std::lock_guard<std::mutex> lk(mu);
+  return known[key] = device_info(device).sms * per_sm;
 }
 
 template <class R, int M, bool ADJ>
@@ -480,7 +484,7 @@ int standalone_adjoint(vqc_state h, void* lam, void* y, const GateSpec& gs, bool
 
 // The structure class of a one-qubit matrix (exact zeros: the matrices are
 // built from closed forms, so structural zeros are exact).
-static int u1_form(const std::vector<cd>& m) {
+static int u1_form(const Mat& m) {
   const cd u00 = m[0], u01 = m[1], u10 = m[2], u11 = m[3];
   if (u00 == cd(0) && u11 == cd(0) && u01 == cd(1) && u10 == cd(1)) return kFormSwap;
   if (u01 == cd(0) && u10 == cd(0)) return kFormDiag;
@@ -568,11 +572,16 @@ static double pass_fma_ops(const PlanPass& p, int n, bool adj) {
 // The controls of an op by place: qubits outside the tile (one test per tile),
 // thread bits (one test per op), register bits (rc, and the amplitudes they
 // enable in rmask).
-static void place_controls(DevOp& o, uint64_t cmask, uint64_t cval, int n, uint64_t tile_mask,
-                           std::map<int, int>& tbit, const std::vector<int>& rs, std::vector<std::pair<int, int>>& rc) {
-  for (int q = 0; q < n; ++q) {
-    if (!(cmask >> q & 1)) continue;
-    const int v = (int)(cval >> q & 1);
+struct RegCtl {  // register controls: (j-bit, value)
+  int n = 0;
+  std::pair<int, int> c[8];
+  const std::pair<int, int>* begin() const { return c; }
+  const std::pair<int, int>* end() const { return c + n; }
+};
+static void place_controls(DevOp& o, uint64_t cmask, uint64_t cval, uint64_t tile_mask, const int (&tbit)[64],
+                           const std::vector<int>& rs, RegCtl& rc) {
+  for (uint64_t m = cmask; m; m &= m - 1) {
+    const int q = __builtin_ctzll(m), v = (int)(cval >> q & 1);
     if (!(tile_mask >> q & 1)) {
       o.gmask |= 1ull << q;
       if (v) o.gval |= 1ull << q;
@@ -580,18 +589,16 @@ static void place_controls(DevOp& o, uint64_t cmask, uint64_t cval, int n, uint6
     }
     const int b = tbit[q], j = (int)(std::find(rs.begin(), rs.end(), b) - rs.begin());
     if (j < (int)rs.size()) {
-      rc.push_back({j, v});
+      rc.c[rc.n++] = {j, v};
     } else {
       o.cmask |= 1u << b;
       if (v) o.cval |= 1u << b;
     }
   }
-  uint32_t rmask = 0;
-  for (uint32_t j = 0; j < (1u << rs.size()); ++j) {
-    bool ok = true;
-    for (auto& c : rc) ok = ok && ((int)(j >> c.first & 1) == c.second);
-    if (ok) rmask |= 1u << j;
-  }
+  uint32_t need = 0, val = 0, rmask = 0;
+  for (auto& c : rc) need |= 1u << c.first, val |= (uint32_t)c.second << c.first;
+  for (uint32_t j = 0; j < (1u << rs.size()); ++j)
+    if ((j & need) == val) rmask |= 1u << j;
   o.rmask = (int32_t)rmask;
   if (o.cmask) o.code |= kCodeCtl;
   if (o.gmask) o.code |= kCodeGCtl;
@@ -599,17 +606,50 @@ static void place_controls(DevOp& o, uint64_t cmask, uint64_t cval, int n, uint6
 
 // Tile bits of the warp index (thread bits 5 and up) in a stage's layout.
 static uint32_t warp_bits(const PlanStage& st, int M) {
-  uint32_t m = 0;
-  for (int b = 0, i = 0; b < M; ++b)
-    if (std::find(st.rs.begin(), st.rs.end(), b) == st.rs.end() && i++ >= 5) m |= 1u << b;
-  return m;
+  uint32_t rest = (1u << M) - 1;
+  for (int b : st.rs) rest &= ~(1u << b);
+  for (int i = 0; i < 5; ++i) rest &= rest - 1;
+  return rest;
 }
+
+// A stage's index tables: global offsets of tile indices by bit, and the
+// thread's nibble tables by doubling (thr: its tile bits, ascending).
+struct StageTables {
+  int64_t g[16];
+  int thr[16], nthr = 0;
+  StageTables(const PlanPass& p, int M, uint32_t rsmask) {
+    for (int b = 0; b < M; ++b) {
+      g[b] = int64_t(1) << p.tile_q[b];
+      if (!(rsmask >> b & 1)) thr[nthr++] = b;
+    }
+  }
+  int64_t global(uint32_t t) const {
+    int64_t r = 0;
+    for (; t; t &= t - 1) r |= g[__builtin_ctz(t)];
+    return r;
+  }
+  template <class Put>
+  void nibbles(Put put) const {
+    for (int k = 0; k < 2; ++k) {
+      uint32_t t[16] = {0};
+      int64_t gt[16] = {0};
+      put(k, 0, 0u, int64_t(0));
+      for (int i = 0; i < 4; ++i)
+        for (int nib = 1 << i; nib < 2 << i; ++nib) {
+          const int low = nib ^ (1 << i);
+          const bool on = 4 * k + i < nthr;
+          t[nib] = t[low] | (on ? 1u << thr[4 * k + i] : 0u);
+          gt[nib] = gt[low] | (on ? g[thr[4 * k + i]] : 0);
+          put(k, nib, t[nib], gt[nib]);
+        }
+    }
+  }
+};
 
 // One stage of the FP32 (packed) tile body: its DevStageF tables, its ops
 // (j-bit targets, register controls as compile-time cases or a mask, the
 // coefficient layouts of tile_f32.cuh) and their pool blocks.
-static void stage_f32(const PlanPass& p, const PlanStage& st, int M, int n, uint64_t tile_mask,
-                      std::map<int, int>& tbit, bool adj, int& slot, int row, std::vector<DevStageF>& ds,
+static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t tile_mask, const int (&tbit)[64], bool adj, int& slot, int row, std::vector<DevStageF>& ds,
                       std::vector<DevOp>& dops, std::vector<float2>& pool, size_t pool_begin,
                       std::vector<AccRef>* accs, int rb) {
   DevStageF s{};
@@ -625,27 +665,15 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, int n, uint
     dep[j] = t;
     s.dep[j] = t;
   }
-  std::vector<int> thr;
-  for (int b = 0; b < M; ++b)
-    if (!(rsmask >> b & 1)) thr.push_back(b);
-  auto gq = [&](uint32_t t) {
-    int64_t g = 0;
-    for (int b = 0; b < M; ++b)
-      if (t >> b & 1) g |= int64_t(1) << p.tile_q[b];
-    return g;
-  };
-  for (int k = 0; k < 2; ++k)
-    for (int nib = 0; nib < 16; ++nib) {
-      uint32_t t = 0;
-      for (int i = 0; i < 4; ++i)
-        if ((nib >> i & 1) && 4 * k + i < (int)thr.size()) t |= 1u << thr[4 * k + i];
-      s.thr[k][nib] = t;
-      s.swt[k][nib] = f32t::swz_pair(t >> 1);
-      s.gthr[k][nib] = gq(t);
-    }
+  const StageTables tabs(p, M, rsmask);
+  tabs.nibbles([&](int k, int nib, uint32_t t, int64_t g) {
+    s.thr[k][nib] = t;
+    s.swt[k][nib] = f32t::swz_pair(t >> 1);
+    s.gthr[k][nib] = g;
+  });
   for (int m = 0; m < np; ++m) {
     s.swm[m] = f32t::swz_pair(dep[2 * m] >> 1);
-    s.gdep[m] = gq(dep[2 * m]);
+    s.gdep[m] = tabs.global(dep[2 * m]);
   }
   auto jbit = [&](int b) { return (int)(std::find(rs.begin(), rs.end(), b) - rs.begin()); };
   auto put = [&](double a, double b) { pool.push_back(make_float2((float)a, (float)b)); };
@@ -656,10 +684,10 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, int n, uint
     DevOp o{};
     o.code = f.kind;
     o.slot = -1;
-    std::vector<std::pair<int, int>> rc;  // register controls: (j-bit, value)
-    place_controls(o, f.cmask, f.cval, n, tile_mask, tbit, rs, rc);
+    RegCtl rc;
+    place_controls(o, f.cmask, f.cval, tile_mask, tbit, rs, rc);
     int rctl = 0;
-    if (!rc.empty()) rctl = (rc.size() == 1 && rc[0].second == 1) ? rc[0].first + 1 : 7;
+    if (rc.n) rctl = (rc.n == 1 && rc.c[0].second == 1) ? rc.c[0].first + 1 : 7;
     while (pool.size() % 2) put(0, 0);  // each op's block starts on 16 bytes
     o.mat = (int)(pool.size() - pool_begin);
     if (f.kind == kOpU1) {
@@ -729,10 +757,10 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, int n, uint
         DevOp a = o;
         a.code = (a.code & ~15) | kOpAccD;
         dops.push_back(a);
-        if (accs) accs->push_back(AccRef{row + o.slot, f});
+        if (accs) accs->push_back(AccRef{row + o.slot, f.grads});
         continue;
       }
-      if (accs) accs->push_back(AccRef{row + o.slot, f, (o.code & kCodeAH) != 0});
+      if (accs) accs->push_back(AccRef{row + o.slot, f.grads, (o.code & kCodeAH) != 0});
       o.code |= kCodeAcc;
     }
     dops.push_back(o);
@@ -759,8 +787,8 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
     plan_stages(p, M, dtype, packed, rb);
     std::vector<DevStage> ds;
     std::vector<DevOp> dops;
-    std::map<int, int> tbit;
-    for (int b = 0; b < M; ++b) tbit[p.tile_q[b]] = b;
+    int tbit[64];
+    tile_bits(p, tbit);
     uint64_t tile_mask = 0;
     for (int q : p.tile_q) tile_mask |= 1ull << q;
     int slot = 0;
@@ -770,39 +798,27 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
     for (const PlanStage& st : p.stages) {
       if constexpr (std::is_same<R, float>::value) {
         if (packed) {
-          stage_f32(p, st, M, n, tile_mask, tbit, ADJ, slot, row, dsf, dops, pool, pool_begin, accs, rb);
+          stage_f32(p, st, M, tile_mask, tbit, ADJ, slot, row, dsf, dops, pool, pool_begin, accs, rb);
           continue;
         }
       }
       DevStage s{};
       uint32_t rsmask = 0;
       for (int b : st.rs) rsmask |= 1u << b;
-      std::vector<int> thr;
-      for (int b = 0; b < M; ++b)
-        if (!(rsmask >> b & 1)) thr.push_back(b);
-      auto gq = [&](uint32_t t) {
-        int64_t g = 0;
-        for (int b = 0; b < M; ++b)
-          if (t >> b & 1) g |= int64_t(1) << p.tile_q[b];
-        return g;
-      };
+      const StageTables tabs(p, M, rsmask);
       for (int j = 0; j < 16; ++j) {
         uint32_t t = 0;
         for (int i = 0; i < kRegBits; ++i)
           if (j >> i & 1) t |= 1u << st.rs[i];
         s.dep[j] = t;
         s.swm[j] = Swz<R>::f(t);
-        s.gdep[j] = gq(t);
+        s.gdep[j] = tabs.global(t);
       }
-      for (int k = 0; k < 2; ++k)
-        for (int nib = 0; nib < 16; ++nib) {
-          uint32_t t = 0;
-          for (int i = 0; i < 4; ++i)
-            if ((nib >> i & 1) && 4 * k + i < (int)thr.size()) t |= 1u << thr[4 * k + i];
-          s.thr[k][nib] = t;
-          s.swt[k][nib] = Swz<R>::f(t);
-          s.gthr[k][nib] = gq(t);
-        }
+      tabs.nibbles([&](int k, int nib, uint32_t t, int64_t g) {
+        s.thr[k][nib] = t;
+        s.swt[k][nib] = Swz<R>::f(t);
+        s.gthr[k][nib] = g;
+      });
       s.cta = warp_bits(st, M) != warp_bits(p.stages[(&st - p.stages.data() + 1) % p.stages.size()], M);
       s.op_begin = (int)dops.size();
       for (int oi : st.ops) {
@@ -818,12 +834,12 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
           cm |= 1ull << f.dq[i];
           if (k0 >> i & 1) cv |= 1ull << f.dq[i];
         }
-        std::vector<std::pair<int, int>> rc;
-        place_controls(o, cm, cv, n, tile_mask, tbit, st.rs, rc);
+        RegCtl rc;
+        place_controls(o, cm, cv, tile_mask, tbit, st.rs, rc);
         int sel = k0 < 0 ? kSelDiag : (f.mat[k0] == cd(-1) ? kSelFlip : kSelPhase);
         if (f.kind == kOpU1) {
           const int r = slot_of(tbit[f.tq[0]]), form = u1_form(f.mat);
-          sel = kSelU1 + (r | (rc.empty() ? 0 : 4) | form << 3);
+          sel = kSelU1 + (r | (rc.n ? 4 : 0) | form << 3);
           if (ADJ && f.acc) o.code |= (acc_kind(f) << 14) | (acc_anti_hermitian(f) ? kCodeAH : 0);
         }
         if (f.kind == kOpU2) sel = kSelU2 + slot_of(tbit[f.tq[0]]) * 4 + slot_of(tbit[f.tq[1]]);
@@ -874,10 +890,10 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
             a.cmask = a.cval = 0;
             a.gmask = a.gval = 0;
             dops.push_back(a);
-            if (accs) accs->push_back(AccRef{row + o.slot, f});
+            if (accs) accs->push_back(AccRef{row + o.slot, f.grads});
             continue;
           }
-          if (accs) accs->push_back(AccRef{row + o.slot, f, (o.code & kCodeAH) != 0});
+          if (accs) accs->push_back(AccRef{row + o.slot, f.grads, (o.code & kCodeAH) != 0});
           o.code |= kCodeAcc;
         }
         dops.push_back(o);
@@ -1181,8 +1197,9 @@ static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const do
   int rc = reserve_ops(h, bound);
   if (rc) return rc;
   size_t off = 0, take = 1;
-  for (size_t first = 0; first < passes.size(); first += take, take *= 2) {
-    const size_t last = std::min(passes.size(), first + take);
+  const uint64_t compiles = jit_compiles();
+  for (size_t first = 0, last; first < passes.size(); first = last, take *= 2) {
+    last = jit_compiles() != compiles ? passes.size() : std::min(passes.size(), first + take);
     std::vector<PlanPass> chunk(std::make_move_iterator(passes.begin() + first),
                                 std::make_move_iterator(passes.begin() + last));
     size_t used = 0;
@@ -1239,8 +1256,9 @@ static std::vector<PItem> reverse_items(const std::vector<GateSpec>& specs,
         const int d = 1 << gs.k;
         for (const ParamInfo& pi : params[i]) {
           PGrad pg{pi.index, {}};
-          for (int j = 0; j < d; ++j) pg.D.push_back(pi.D[(size_t)j * d + j]);
-          f.grads.push_back(pg);
+          pg.D.assign(d, cd(0));
+          for (int j = 0; j < d; ++j) pg.D[j] = pi.D[(size_t)j * d + j];
+          f.grads.push_back(std::move(pg));
         }
       } else {
         ok = false;
@@ -1280,8 +1298,11 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
   }
   // run pass by pass so that standalone gates with parameters see the right states
   const uint64_t call = new_call();
-  std::vector<PlanPass> one(1);
   int row_base = 0;
+  const uint64_t compiles = jit_compiles();
+  size_t bound = 256, off = 0, take = 1;
+  for (const PlanPass& p : passes) bound += op_bytes_bound<R>(p) + sizeof(RedItem) + 256;
+  if (int rc = reserve_ops(h, bound)) return rc;
   for (size_t pi = 0; pi < passes.size(); ++pi) {
     if (passes[pi].standalone) {
       const int gi = passes[pi].gate;
@@ -1295,13 +1316,19 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
       }
       continue;
     }
-    // group consecutive tile passes into one upload
+    // consecutive tile passes in chunks of 1, 2, 4, ... passes, each in its own
+    // region of the op buffer (as the forward sweep): the device starts on the
+    // first while the host serialises the rest
     size_t pj = pi;
     std::vector<PlanPass> group;
-    while (pj < passes.size() && !passes[pj].standalone) group.push_back(std::move(passes[pj++]));
+    if (jit_compiles() != compiles) take = passes.size();
+    while (pj < passes.size() && !passes[pj].standalone && group.size() < take) group.push_back(std::move(passes[pj++]));
+    take *= 2;
     std::vector<AccRef> gaccs;
-    int rc = run_plan<R, M, true>(h, y, lam, group, specs, &gaccs, h->accbuf + (size_t)row_base * 8, call);
+    size_t used = 0;
+    int rc = run_plan<R, M, true>(h, y, lam, group, specs, &gaccs, h->accbuf + (size_t)row_base * 8, call, off, &used);
     if (rc) return rc;
+    off = (off + used + 255) & ~size_t(255);
     for (auto& a : gaccs) {
       a.row += row_base;
       accs.push_back(std::move(a));
@@ -1342,13 +1369,13 @@ void contract_grads(const std::vector<AccRef>& accs, const double* A, double* gr
     const double* r = &A[(size_t)a.row * 8];
     if (a.ah) {
       // r = (Im A00, Im A11, Re A01 - Re A10, Im A01 + Im A10), D anti-Hermitian
-      for (const PGrad& pg : a.op.grads)
+      for (const PGrad& pg : a.grads)
         grads[pg.param] = -pg.D[0].imag() * r[0] - pg.D[3].imag() * r[1] + pg.D[1].real() * r[2] -
                           pg.D[1].imag() * r[3];
       continue;
     }
     const cd Av[4] = {cd(r[0], r[1]), cd(r[2], r[3]), cd(r[4], r[5]), cd(r[6], r[7])};
-    for (const PGrad& pg : a.op.grads) {
+    for (const PGrad& pg : a.grads) {
       double g = 0;
       for (size_t i = 0; i < pg.D.size() && i < 4; ++i) g += (pg.D[i] * Av[i]).real();
       grads[pg.param] = g;

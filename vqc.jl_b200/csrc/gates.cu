@@ -15,7 +15,7 @@
 
 namespace vqc {
 
-int order_matrix(int n, int k, const int* pos, const double* mat, int* sp, std::vector<cd>& M) {
+int order_matrix(int n, int k, const int* pos, const double* mat, int* sp, Mat& M) {
   if (k < 1) return fail(VQC_ERR_ARG, "gate needs at least one position");
   if (k > 5) return fail(VQC_ERR_UNSUPPORTED, "only implement 5-qubit gates and less currently.");
   if (!pos || !mat) return fail(VQC_ERR_ARG, "null positions or matrix");
@@ -57,10 +57,14 @@ int analyze_gate(int n, int k, const int* pos, const double* mat, bool dagger, G
     if (!std::isfinite(g.U[i].real()) || !std::isfinite(g.U[i].imag()))
       return fail(VQC_ERR_ARG, "gate matrix has a non-finite entry");
   if (dagger) {
-    std::vector<cd> T((size_t)d * d);
-    for (int r = 0; r < d; ++r)
-      for (int c = 0; c < d; ++c) T[(size_t)r * d + c] = std::conj(g.U[(size_t)c * d + r]);
-    g.U.swap(T);
+    for (int r = 0; r < d; ++r) {
+      g.U[(size_t)r * d + r] = std::conj(g.U[(size_t)r * d + r]);
+      for (int c = 0; c < r; ++c) {
+        const cd t = std::conj(g.U[(size_t)r * d + c]);
+        g.U[(size_t)r * d + c] = std::conj(g.U[(size_t)c * d + r]);
+        g.U[(size_t)c * d + r] = t;
+      }
+    }
   }
   g.ns = 0;
   for (int j = 0; j < d; ++j) {

@@ -550,6 +550,10 @@ namespace {
 thread_local int t_thread_cap = 0;
 }
 void jit_set_thread_cap(int n) { t_thread_cap = n < 0 ? 0 : n; }
+namespace {
+thread_local uint64_t t_compiles = 0;
+}
+uint64_t jit_compiles() { return t_compiles; }
 
 int jit_kernels(const std::vector<std::string>& srcs, std::vector<const void*>& out, const char* name) {
   out.assign(srcs.size(), nullptr);
@@ -613,6 +617,7 @@ int jit_kernels(const std::vector<std::string>& srcs, std::vector<const void*>& 
       if (it != cache().end() && !it->second.failed) out[i] = (const void*)it->second.kernel;
     }
     prof_note("jit_compiled_passes", (long long)todo.size());
+    t_compiles += todo.size();
   }
   return VQC_OK;
 }

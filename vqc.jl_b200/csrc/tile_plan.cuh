@@ -25,7 +25,7 @@ struct Swz<double> {  // 16-byte amplitudes: quarter-warps must hit 8 distinct 1
 
 struct PGrad {
   int param;             // caller's parameter index
-  std::vector<cd> D;     // U1: 2x2 over the target (control subspace); AccD: 2^nd diagonal bins
+  Mat2 D;                // U1: 2x2 over the target (control subspace); AccD: 2^nd diagonal bins
 };
 
 struct FOp {
@@ -33,7 +33,7 @@ struct FOp {
   int tq[2] = {-1, -1};  // target qubits (ascending)
   uint64_t cmask = 0, cval = 0;  // control qubits and their firing values (global bits)
   uint64_t qubits = 0;   // every qubit the op reads or writes
-  std::vector<cd> mat;   // U1 2x2, U2 4x4 (bit 0 <-> tq[0]), diagonal 2^nd table
+  Mat mat;               // U1 2x2, U2 4x4 (bit 0 <-> tq[0]), diagonal 2^nd table
   int nd = 0;
   int dq[5] = {0, 0, 0, 0, 0};
   bool acc = false;
@@ -49,7 +49,7 @@ struct PassShape {
 // reduced matrix A) its partial sums land in.
 struct AccRef {
   int row;
-  FOp op;
+  std::vector<PGrad> grads;
   bool ah = false;  // the row holds the anti-Hermitian projection (kAccAH)
 };
 
@@ -144,6 +144,10 @@ std::string jit_pass_source(int M, bool adj, const DevStageF* stages, int nstage
 // host core).  A background compiler sets a few so the threads that plan and
 // launch keep their cores.
 void jit_set_thread_cap(int n);
+// Kernels compiled so far in calls of this thread.  A sweep launched in chunks
+// that meets a missing kernel takes the rest as one chunk, so that its other
+// missing kernels compile in parallel.
+uint64_t jit_compiles();
 // Kernels for the given pass sources (nullptr for an empty source or a failed compile).
 int jit_kernels(const std::vector<std::string>& srcs, std::vector<const void*>& out, const char* name = "vqc_pass");
 // A serialised pass for jit_pass_kernels (stages == nullptr: not a tile pass).
