@@ -25,7 +25,6 @@ int pauli_run(vqc_state h, const void* bra, const void* ket, void* out, const vq
               bool write, bool acc, bool hermitian_part, double* result, bool* deferred = nullptr);
 int expect_dense_device(vqc_state h, const void* bra, const void* ket, int k, const int* sp, const Mat& M,
                         double* res);
-int apply_circuit_raw(vqc_state h, const vqc_gate* gates, int ngates, const double* mats, bool dm, int fuse);
 
 constexpr int kAccMaxS = 4;  // A is reduced in one pass for |S| <= 4
 
@@ -255,7 +254,7 @@ int vqc_adjoint_grad(vqc_state psi0, const vqc_gate* gates, int ngates, const do
   // forward: y = circuit * psi0 (run on a view of psi0's handle whose buffer is y)
   void* keep = psi0->d;
   psi0->d = y;
-  rc = apply_circuit_raw(psi0, gates, ngates, mats, false, 1);
+  rc = apply_circuit_fused(psi0, gates, ngates, mats, psi0->dtype == VQC_C128);
   psi0->d = keep;
   if (rc) return rc;
   // E = <y|H|y>; cotangent lam = (conj(z) H + z H^dagger) y with z = 1.  E

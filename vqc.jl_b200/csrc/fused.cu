@@ -175,6 +175,7 @@ struct PlanPass {
   std::vector<FOp> ops;
   std::vector<PlanStage> stages;
   int nslots = 0;
+  double norm0 = 1;              // the deferred norm when the pass starts (defer_phases)
 };
 
 static void tile_bits(const PlanPass& p, int (&tbit)[64]) {
@@ -283,6 +284,146 @@ static void plan_passes(int n, const TileConfig& tc, bool adj, std::vector<PItem
   }
 }
 
+// Phases deferred.  A 2x2 M with |m00| = |m11| is a diag(1, p) T, a = m00, |p| = 1,
+// T = [[1, x], [y, 1]], and T takes half the products of a general 2x2 (8
+// instead of 16 FMAs per pair of amplitudes); the tile passes are bound by their
+// arithmetic.  The phase p stays behind as a pending diag(1, p) on the qubit and
+// a as a factor g of the whole state.  A pending phase passes a control and a
+// diagonal gate unchanged, turns another gate on its qubit into one with rotated
+// off-diagonal entries, and is absorbed by the next uncontrolled one-qubit gate
+// there; the last such gate (before the end of the circuit, or a gate outside
+// the tile passes) takes its whole matrix and g, so no pass is added.  The first
+// deferred gate of a pass takes the norm of g (real diagonal, 12 FMAs), so that
+// amplitudes grow over one pass only.  With U3 + CZ every dense gate but the last
+// layer's costs half; with CRX ladders the controlled gates cost 6 instead of 4
+// per pair, the merged rotations 8 instead of 16.
+//
+// Which form a gate takes depends on its place alone, not on its angle (but for
+// |m00| < kMinPivot and exact zeros), so that new angles reuse compiled passes.
+// T is a multiple of a unitary whatever |x|: a large x is as accurate as a small one.
+//
+// Only where the passes are compiled (states of 2^18 FP32, 2^20 FP64 amplitudes
+// and more): the interpreted ones are bound by latency, and a CNOT that was a
+// swap of two loads becomes a product (serving's reverse launches 66 -> 81 us).
+// Measured: reverse pass 1,060 -> 957 us and forward 350 -> 325 us at 2^26 FP32,
+// U3 + CZ + Toffoli pass 7.9 -> 5.6 ms at 2^30 FP32 and 2.3 -> 1.75 ms at 2^27 FP64.
+// Accuracy against FP64 (16 circuits of 20 layers on 20 qubits, FP32): gradient
+// 5.6e-7 (1.04e-6 with whole matrices), norm 1.4e-7 (3.1e-7), energy as before
+// (1.7e-7, 2.0e-7 absolute): the rounding of the angles, not of the amplitudes,
+// decides it.  The FP32 gradient's own forward sweep keeps whole matrices (its
+// passes gain 2 % of the gradient's time), so that sweep's energy is unchanged.
+// In FP32 x is rounded first and y = -conj(x), so that this holds exactly.
+//
+// The reverse sweep applies the same ops to both states, so its reduced
+// matrices come out in the pending frame: A[a][b] = |g|^2 conj(p_a) p_b A'[a][b]
+// over the op's target.  The phases are folded into the D matrices here; |g| is
+// the product over the ops that have run, in the order of the pass's stages
+// (AccRef::scale).
+constexpr double kMinPivot = 1e-9, kMinScale = 1e-15;  // (amplitudes grow by 1 / |g|)
+// A phase within rounding of 1, i, -1 or -i is that one (a rounding error must
+// not decide which form the next gates take).
+static cd whole_turns(cd p) {
+  for (const cd& q : {cd(1), cd(-1), cd(0, 1), cd(0, -1)})
+    if (std::abs(p - q) < 1e-14) return q;
+  return p;
+}
+static void defer_phases(int n, bool adj, bool f32, std::vector<PlanPass>& passes) {
+  for (const PlanPass& p : passes)
+    if (adj && p.standalone) return;  // (their reduced matrices are taken in the plain frame)
+  // the ops on each qubit that a later uncontrolled one-qubit op follows
+  std::vector<char> later;  // by op, in order
+  {
+    std::vector<char> open(n, 0);
+    size_t total = 0;
+    for (const PlanPass& p : passes) total += p.ops.size();
+    later.assign(total, 0);
+    size_t k = total;
+    for (size_t pi = passes.size(); pi-- > 0;) {
+      const PlanPass& p = passes[pi];
+      if (p.standalone) {
+        std::fill(open.begin(), open.end(), 0);
+        continue;
+      }
+      for (size_t i = p.ops.size(); i-- > 0;) {
+        const FOp& f = p.ops[i];
+        --k;
+        if (f.kind != kOpU1 || f.cmask) continue;
+        later[k] = open[f.tq[0]];
+        open[f.tq[0]] = 1;
+      }
+    }
+  }
+  std::vector<cd> ph(n, cd(1));
+  cd g(1);
+  size_t k = 0;
+  auto in_frame = [&](FOp& f) {  // the reduced matrix's frame, after the op
+    if (!adj || !f.acc || f.kind != kOpU1) return;
+    const cd p = ph[f.tq[0]];
+    if (p != cd(1))
+      for (PGrad& pg : f.grads) pg.D[1] *= p, pg.D[2] *= std::conj(p);
+  };
+  for (PlanPass& pass : passes) {
+    bool first = true;  // no deferred gate in this pass yet
+    pass.norm0 = std::abs(g);
+    for (FOp& f : pass.ops) {
+      const double before = std::abs(g);
+      const bool absorbed = later[k++];
+      if (f.kind == kOpU2) {
+        const cd a = ph[f.tq[0]], b = ph[f.tq[1]];
+        if (a != cd(1) || b != cd(1)) {
+          const cd c[4] = {cd(1), a, b, a * b};
+          for (int r = 0; r < 4; ++r)
+            for (int q = 0; q < 4; ++q)
+              if (f.mat[4 * r + q] != cd(0)) f.mat[4 * r + q] *= c[q] * std::conj(c[r]);
+        }
+      } else if (f.kind == kOpU1) {
+        cd& p = ph[f.tq[0]];
+        Mat& m = f.mat;
+        if (f.cmask) {
+          if (p != cd(1)) {
+            if (m[1] != cd(0)) m[1] *= p;
+            if (m[2] != cd(0)) m[2] *= std::conj(p);
+          }
+        } else {
+          if (p != cd(1)) m[1] *= p, m[3] *= p;
+          const cd a = m[0];
+          const double na = std::abs(a), nb = std::abs(m[3]);
+          const double top = std::max(std::max(na, nb), std::max(std::abs(m[1]), std::abs(m[2])));
+          if (absorbed && std::min(na, nb) > kMinPivot * top && std::abs(na - nb) <= 1e-13 * top) {
+            const cd np = whole_turns((m[3] / nb) * std::conj(a / na));
+            cd x = m[1] / a, y = m[2] / (a * np);
+            double s = 1;
+            if (f32 && std::abs(y + std::conj(x)) <= 1e-13 * (1 + std::abs(x))) {
+              const cd xr((float)x.real(), (float)x.imag());
+              s = std::sqrt((1 + std::norm(x)) / (1 + std::norm(xr)));
+              x = xr;
+              y = -std::conj(xr);
+            }
+            p = np;
+            g *= a * s;
+            const double ng = std::abs(g);
+            if (first || ng < kMinScale) {
+              m = {cd(ng), ng * x, ng * y, cd(ng)};
+              g /= ng;
+              f.form = kFormRC;
+            } else {
+              m = {cd(1), x, y, cd(1)};
+              f.form = x == cd(0) && y == cd(0) ? kFormId : kFormUD;
+            }
+            first = false;
+          } else {
+            for (cd& v : m) v *= g;
+            g = cd(1);
+            p = cd(1);
+          }
+        }
+      }
+      in_frame(f);
+      f.gain = std::abs(g) / before;
+    }
+  }
+}
+
 // Conflict check of a register-bit set for the shared-memory swizzle.
 // FP64: 16-byte amplitudes, quarter-warps over the tile swizzle Swz<double>;
 // FP32: 8-byte amplitudes, half-warps over Swz<float>.  Packed FP32: 16-byte
@@ -379,6 +520,14 @@ static void plan_stages(PlanPass& p, int M, int dtype, bool packed, int rb = kRe
     p.stages.push_back(std::move(st));
     pending.swap(rest);
   }
+}
+
+// Tile bits of the warp index (thread bits 5 and up) in a stage's layout.
+static uint32_t warp_bits(const PlanStage& st, int M, int rb = kRegBits) {
+  uint32_t rest = (1u << M) - 1;
+  for (int b : st.rs) rest &= ~(1u << b);
+  for (int i = 0; i < std::min(5, M - rb); ++i) rest &= rest - 1;
+  return rest;
 }
 
 // ----------------------------------------------------------------------------- execution
@@ -485,13 +634,16 @@ int standalone_adjoint(vqc_state h, void* lam, void* y, const GateSpec& gs, bool
 // The structure class of a one-qubit matrix (exact zeros: the matrices are
 // built from closed forms, so structural zeros are exact).
 static int u1_form(const Mat& m) {
-  const cd u00 = m[0], u01 = m[1], u10 = m[2], u11 = m[3];
-  if (u00 == cd(0) && u11 == cd(0) && u01 == cd(1) && u10 == cd(1)) return kFormSwap;
-  if (u01 == cd(0) && u10 == cd(0)) return kFormDiag;
+  const cd u00 = m[0], u01 = m[1], u10 = m[2], u11 = m[3], one(1), zero(0);
+  const bool diag = u01 == zero && u10 == zero, off = u00 == zero && u11 == zero;
+  if (diag) return u00 == one && u11 == one ? kFormId : kFormDiag;
+  if (off) return u01 == one && u10 == one ? kFormSwap : kFormOff;
   if (u00.imag() == 0 && u01.imag() == 0 && u10.imag() == 0 && u11.imag() == 0) return kFormReal;
   if (u00.imag() == 0 && u11.imag() == 0 && u01.real() == 0 && u10.real() == 0) return kFormRI;
+  if (u00.imag() == 0 && u11.imag() == 0) return kFormRC;
   return kFormGen;
 }
+static int u1_form(const FOp& f) { return f.form >= 0 ? f.form : u1_form(f.mat); }
 
 // Which entries of the reduced matrix the op's parameters need.
 static int acc_kind(const FOp& f) {
@@ -533,8 +685,8 @@ static int single_entry(const FOp& f) {
 
 // FMA-pipe lane operations (fused multiply-adds, multiplies, adds) of one pass
 // over the whole state of n qubits, as the tile bodies implement its ops: a
-// one-qubit op costs per amplitude pair and state 16 (general form), 8
-// (RX-like, real, diagonal) or 0 (swap), and in the reverse sweep its
+// one-qubit op costs per amplitude pair and state 16 (general form), 12 (real
+// diagonal), 8 (the other structured forms) or 0 (swap, identity), and in the reverse sweep its
 // reduced-matrix accumulation 16 / 8 per pair (12 / 8 / 4 for the
 // anti-Hermitian projection); a two-qubit op 64 per amplitude quad and state;
 // a diagonal op 4 per state and amplitude that an entry other than 1 touches
@@ -544,12 +696,12 @@ static int single_entry(const FOp& f) {
 static double pass_fma_ops(const PlanPass& p, int n, bool adj) {
   const double pairs = std::ldexp(1.0, n - 1), amps = std::ldexp(1.0, n);
   const int nst = adj ? 2 : 1;
-  static const int per_pair[5] = {16, 8, 8, 8, 0};  // by kForm*
+  static const int per_pair[kForms] = {16, 8, 8, 8, 0, 8, 12, 8, 0};  // by kForm*
   double ops = 0;
   for (const FOp& f : p.ops) {
     const double act = std::ldexp(1.0, -popc64(f.cmask));
     if (f.kind == kOpU1) {
-      double o = (double)per_pair[u1_form(f.mat)] * nst;
+      double o = (double)per_pair[u1_form(f)] * nst;
       if (adj && f.acc) {
         const int k = acc_kind(f);
         if (acc_anti_hermitian(f))
@@ -604,14 +756,6 @@ static void place_controls(DevOp& o, uint64_t cmask, uint64_t cval, uint64_t til
   if (o.gmask) o.code |= kCodeGCtl;
 }
 
-// Tile bits of the warp index (thread bits 5 and up) in a stage's layout.
-static uint32_t warp_bits(const PlanStage& st, int M) {
-  uint32_t rest = (1u << M) - 1;
-  for (int b : st.rs) rest &= ~(1u << b);
-  for (int i = 0; i < 5; ++i) rest &= rest - 1;
-  return rest;
-}
-
 // A stage's index tables: global offsets of tile indices by bit, and the
 // thread's nibble tables by doubling (thr: its tile bits, ascending).
 struct StageTables {
@@ -649,7 +793,7 @@ struct StageTables {
 // One stage of the FP32 (packed) tile body: its DevStageF tables, its ops
 // (j-bit targets, register controls as compile-time cases or a mask, the
 // coefficient layouts of tile_f32.cuh) and their pool blocks.
-static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t tile_mask, const int (&tbit)[64], bool adj, int& slot, int row, std::vector<DevStageF>& ds,
+static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t tile_mask, const int (&tbit)[64], bool adj, int& slot, double& norm, int row, std::vector<DevStageF>& ds,
                       std::vector<DevOp>& dops, std::vector<float2>& pool, size_t pool_begin,
                       std::vector<AccRef>* accs, int rb) {
   DevStageF s{};
@@ -678,9 +822,14 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t ti
   auto jbit = [&](int b) { return (int)(std::find(rs.begin(), rs.end(), b) - rs.begin()); };
   auto put = [&](double a, double b) { pool.push_back(make_float2((float)a, (float)b)); };
   auto dup = [&](double a) { put(a, a); };
+  auto dup3 = [&](cd a) { dup(a.real()), dup(a.imag()), dup(-a.imag()); };
+  auto lane3 = [&](cd a, cd b) {
+    put(a.real(), b.real()), put(a.imag(), b.imag()), put(-a.imag(), -b.imag());
+  };
   s.op_begin = (int)dops.size();
   for (int oi : st.ops) {
     const FOp& f = p.ops[oi];
+    norm *= f.gain;
     DevOp o{};
     o.code = f.kind;
     o.slot = -1;
@@ -691,8 +840,8 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t ti
     while (pool.size() % 2) put(0, 0);  // each op's block starts on 16 bytes
     o.mat = (int)(pool.size() - pool_begin);
     if (f.kind == kOpU1) {
-      const int tb = jbit(tbit[f.tq[0]]), form = u1_form(f.mat);
-      o.code |= op_r_bits(tb, 0) | (form << 11) | (rctl << 16);
+      const int tb = jbit(tbit[f.tq[0]]), form = u1_form(f);
+      o.code |= op_r_bits(tb, 0) | form_bits(form) | (rctl << 16);
       if (adj && f.acc) o.code |= (acc_kind(f) << 14) | (acc_anti_hermitian(f) ? kCodeAH : 0);
       const cd u00 = f.mat[0], u01 = f.mat[1], u10 = f.mat[2], u11 = f.mat[3];
       if (tb != 0) {
@@ -711,6 +860,13 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t ti
           case kFormDiag:
             dup(u00.real()), dup(u00.imag()), dup(-u00.imag()), dup(u11.real()), dup(u11.imag()), dup(-u11.imag());
             break;
+          case kFormUD:
+          case kFormOff:
+            dup3(u01), dup3(u10);
+            break;
+          case kFormRC:
+            dup(u00.real()), dup3(u01), dup(u11.real()), dup3(u10);
+            break;
           default: break;
         }
       } else {
@@ -723,6 +879,11 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t ti
           case kFormReal: put(u00.real(), u11.real()), put(u01.real(), u10.real()); break;
           case kFormDiag:
             put(u00.real(), u11.real()), put(u00.imag(), u11.imag()), put(-u00.imag(), -u11.imag());
+            break;
+          case kFormUD:
+          case kFormOff: lane3(u01, u10); break;
+          case kFormRC:
+            put(u00.real(), u11.real()), lane3(u01, u10);
             break;
           default: break;
         }
@@ -757,10 +918,10 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t ti
         DevOp a = o;
         a.code = (a.code & ~15) | kOpAccD;
         dops.push_back(a);
-        if (accs) accs->push_back(AccRef{row + o.slot, f.grads});
+        if (accs) accs->push_back(AccRef{row + o.slot, f.grads, norm * norm});
         continue;
       }
-      if (accs) accs->push_back(AccRef{row + o.slot, f.grads, (o.code & kCodeAH) != 0});
+      if (accs) accs->push_back(AccRef{row + o.slot, f.grads, norm * norm, (o.code & kCodeAH) != 0});
       o.code |= kCodeAcc;
     }
     dops.push_back(o);
@@ -792,13 +953,14 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
     uint64_t tile_mask = 0;
     for (int q : p.tile_q) tile_mask |= 1ull << q;
     int slot = 0;
+    double norm = p.norm0;
     while ((pool.size() * sizeof(cplx<R>)) % 16) pool.push_back(mkc<R>(R(0), R(0)));
     const size_t pool_begin = pool.size();
     std::vector<DevStageF> dsf;
     for (const PlanStage& st : p.stages) {
       if constexpr (std::is_same<R, float>::value) {
         if (packed) {
-          stage_f32(p, st, M, tile_mask, tbit, ADJ, slot, row, dsf, dops, pool, pool_begin, accs, rb);
+          stage_f32(p, st, M, tile_mask, tbit, ADJ, slot, norm, row, dsf, dops, pool, pool_begin, accs, rb);
           continue;
         }
       }
@@ -823,6 +985,7 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
       s.op_begin = (int)dops.size();
       for (int oi : st.ops) {
         const FOp& f = p.ops[oi];
+        norm *= f.gain;
         DevOp o{};
         o.code = f.kind;
         o.slot = -1;
@@ -838,7 +1001,7 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
         place_controls(o, cm, cv, tile_mask, tbit, st.rs, rc);
         int sel = k0 < 0 ? kSelDiag : (f.mat[k0] == cd(-1) ? kSelFlip : kSelPhase);
         if (f.kind == kOpU1) {
-          const int r = slot_of(tbit[f.tq[0]]), form = u1_form(f.mat);
+          const int r = slot_of(tbit[f.tq[0]]), form = u1_form(f);
           sel = kSelU1 + (r | (rc.n ? 4 : 0) | form << 3);
           if (ADJ && f.acc) o.code |= (acc_kind(f) << 14) | (acc_anti_hermitian(f) ? kCodeAH : 0);
         }
@@ -890,10 +1053,10 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
             a.cmask = a.cval = 0;
             a.gmask = a.gval = 0;
             dops.push_back(a);
-            if (accs) accs->push_back(AccRef{row + o.slot, f.grads});
+            if (accs) accs->push_back(AccRef{row + o.slot, f.grads, norm * norm});
             continue;
           }
-          if (accs) accs->push_back(AccRef{row + o.slot, f.grads, (o.code & kCodeAH) != 0});
+          if (accs) accs->push_back(AccRef{row + o.slot, f.grads, norm * norm, (o.code & kCodeAH) != 0});
           o.code |= kCodeAcc;
         }
         dops.push_back(o);
@@ -1159,7 +1322,7 @@ static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& pa
 int fused_supported(vqc_state h) { return h->nq >= kMinTileBits && h->nq <= 40; }
 
 template <class R, int M>
-static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const double* mats) {
+static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const double* mats, bool defer) {
   std::vector<GateSpec> specs(ngates);
   std::vector<PItem> items(ngates);
   // gate analysis, on up to four host threads for long circuits (it precedes
@@ -1184,6 +1347,7 @@ static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const do
       return analyze_gate(h->nq, gates[bad[t]].nq, gates[bad[t]].pos, mats + gates[bad[t]].mat, false, specs[bad[t]]);
   std::vector<PlanPass> passes;
   plan_passes(h->nq, tile_config(h->dtype, h->nq), false, items, passes);
+  if (defer && (use_packed(h) || use_jit64(h))) defer_phases(h->nq, false, h->dtype == VQC_C64, passes);
   const uint64_t call = new_call();
   const char* pc = std::getenv("VQC_PLAN_CHUNKS");  // 0: one serialisation for the whole sweep
   if (passes.size() < 4 || (pc && *pc && std::atoi(pc) == 0))
@@ -1209,7 +1373,7 @@ static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const do
   return VQC_OK;
 }
 
-int apply_circuit_fused(vqc_state h, const vqc_gate* gates, int ngates, const double* mats) {
+int apply_circuit_fused(vqc_state h, const vqc_gate* gates, int ngates, const double* mats, bool defer) {
   if (!fused_supported(h)) {
     for (int i = 0; i < ngates; ++i) {
       int rc = apply_gate_raw(h, gates[i].nq, gates[i].pos, mats + gates[i].mat);
@@ -1218,13 +1382,13 @@ int apply_circuit_fused(vqc_state h, const vqc_gate* gates, int ngates, const do
     return VQC_OK;
   }
   switch (tile_config(h->dtype, h->nq).M + (h->dtype == VQC_C64 ? 0 : 100)) {
-    case 12: return forward_impl<float, 12>(h, gates, ngates, mats);
-    case 11: return forward_impl<float, 11>(h, gates, ngates, mats);
-    case 10: return forward_impl<float, 10>(h, gates, ngates, mats);
-    case 9: return forward_impl<float, 9>(h, gates, ngates, mats);
-    case 111: return forward_impl<double, 11>(h, gates, ngates, mats);
-    case 110: return forward_impl<double, 10>(h, gates, ngates, mats);
-    default: return forward_impl<double, 9>(h, gates, ngates, mats);
+    case 12: return forward_impl<float, 12>(h, gates, ngates, mats, defer);
+    case 11: return forward_impl<float, 11>(h, gates, ngates, mats, defer);
+    case 10: return forward_impl<float, 10>(h, gates, ngates, mats, defer);
+    case 9: return forward_impl<float, 9>(h, gates, ngates, mats, defer);
+    case 111: return forward_impl<double, 11>(h, gates, ngates, mats, defer);
+    case 110: return forward_impl<double, 10>(h, gates, ngates, mats, defer);
+    default: return forward_impl<double, 9>(h, gates, ngates, mats, defer);
   }
 }
 
@@ -1276,6 +1440,7 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
   std::vector<PItem> items = reverse_items(specs, params);
   std::vector<PlanPass> passes;
   plan_passes(h->nq, tile_config(h->dtype, h->nq), true, items, passes);
+  if (use_packed(h) || use_jit64(h)) defer_phases(h->nq, true, h->dtype == VQC_C64, passes);
   // standalone gates with parameters: split their passes out so the per-gate
   // path can evaluate the partials right after the uncompute
   std::vector<AccRef> accs;
@@ -1370,15 +1535,15 @@ void contract_grads(const std::vector<AccRef>& accs, const double* A, double* gr
     if (a.ah) {
       // r = (Im A00, Im A11, Re A01 - Re A10, Im A01 + Im A10), D anti-Hermitian
       for (const PGrad& pg : a.grads)
-        grads[pg.param] = -pg.D[0].imag() * r[0] - pg.D[3].imag() * r[1] + pg.D[1].real() * r[2] -
-                          pg.D[1].imag() * r[3];
+        grads[pg.param] = a.scale * (-pg.D[0].imag() * r[0] - pg.D[3].imag() * r[1] + pg.D[1].real() * r[2] -
+                                     pg.D[1].imag() * r[3]);
       continue;
     }
     const cd Av[4] = {cd(r[0], r[1]), cd(r[2], r[3]), cd(r[4], r[5]), cd(r[6], r[7])};
     for (const PGrad& pg : a.grads) {
       double g = 0;
       for (size_t i = 0; i < pg.D.size() && i < 4; ++i) g += (pg.D[i] * Av[i]).real();
-      grads[pg.param] = g;
+      grads[pg.param] = a.scale * g;
     }
   }
 }
@@ -1430,6 +1595,7 @@ static int build_plan_tm(int n, int dtype, const std::vector<GateSpec>& fspecs, 
   plan_passes(n, tc, false, items, passes);
   for (const PlanPass& p : passes)
     if (p.standalone) return fail(VQC_ERR_UNSUPPORTED, "serving takes gates with at most two target qubits");
+  if (packed) defer_phases(n, false, dtype == VQC_C64, passes);
   serialize_plan<R, M, false>(n, dtype, passes, rp.fwd, nullptr, packed);
   rp.fwd_max = shape_max(rp.fwd);
   if (want_grad) {
@@ -1439,6 +1605,7 @@ static int build_plan_tm(int n, int dtype, const std::vector<GateSpec>& fspecs, 
     for (const PlanPass& p : rpasses)
       if (p.standalone)
         return fail(VQC_ERR_UNSUPPORTED, "serving takes parameterised gates with one target qubit (or diagonal)");
+    if (packed) defer_phases(n, true, dtype == VQC_C64, rpasses);
     serialize_plan<R, M, true>(n, dtype, rpasses, rp.adj, &rp.accs, packed);
     rp.adj_max = shape_max(rp.adj);
   }

@@ -287,7 +287,7 @@ void emit_op(std::ostringstream& os, const DevStageF& st, const DevOp& op, int o
   os << "    { const DevOp* op = x.ops + " << o << ";\n";
   if (gctl) os << "      if ((x.base & op->gmask) == op->gval) {\n";
   if (type == kOpU1) {
-    const int tb = op_r0(code), rctl = (code >> 16) & 7, form = (code >> 11) & 7, kind = acc_kind_of(code);
+    const int tb = op_r0(code), rctl = (code >> 16) & 7, form = form_of(code), kind = acc_kind_of(code);
     const int cb = rctl == 0 ? -1 : rctl - 1;
     os << "      const u64* c = " << cx << " + " << op.mat << ";\n";
     if (ctl) os << "      const bool run = (tthr & op->cmask) == op->cval;\n";
@@ -474,14 +474,15 @@ std::string jit_pass_source(int M, bool adj, const DevStageF* st, int nst, const
 }
 
 // Resident CTAs per SM of the compiled FP64 passes.  Forward: four 128-thread
-// CTAs (128 registers); reverse: VQC_JIT_MINB_ADJ64, default two (255 registers).
+// CTAs (128 registers; three: 2.39 against 2.33 ms per pass at 2^27, five spill:
+// 2.65 ms); reverse: two (255 registers; three at 168: 407 against 337 us at 2^23).
 int jit_min_blocks64(bool adj) { return adj ? env_int("VQC_JIT_MINB_ADJ64", 2) : env_int("VQC_JIT_MINB_FWD64", 4); }
 
 // An FP64 pass written out: the classic plan's stages and ops with the same
 // device functions as the interpreted body (tile_ops.cuh), so both give the
-// same bits.  Interpreting costs 3.4 instructions for every FP64 one on a
-// reverse pass (each op variant leaves the amplitudes in other registers, and
-// every switch moves all of them back), and the FP64 pipe idles at 25 %.
+// same bits.  Measured against the interpreter on 2^23 amplitudes: reverse pass
+// 547 -> 337 us, forward 168 -> 106 us; U3 + CZ + Toffoli on 2^27: 5.0 -> 2.3 ms
+// per pass.  Bound by fetching the straight-line code and by the FP64 pipe.
 std::string jit_pass_source64(int M, bool adj, const DevStage* st, int nst, const DevOp* ops, int npool) {
   if (npool > kJitMaxCoef / 2) return std::string();  // beyond the kernel-parameter space: interpreted
   std::ostringstream os;

@@ -96,7 +96,7 @@ struct alignas(16) DevOp {
 // bits (neither target nor control).
 constexpr int kSelShift = 24;
 __host__ __device__ constexpr int op_free(int code) { return (code >> 16) & 7; }
-enum { kSelU1 = 0, kSelU2 = 64, kSelPhase = 96, kSelFlip = 97, kSelDiag = 98, kSelAccD = 99 };
+enum { kSelU1 = 0, kSelU2 = 96, kSelPhase = 112, kSelFlip = 113, kSelDiag = 114, kSelAccD = 115 };
 constexpr int kCodeCtl = 1 << 8, kCodeGCtl = 1 << 9, kCodeAcc = 1 << 10;
 // r0 / r1 as 3-bit j-bits (the wide FP32 body has j-bits 0..4): bits 4-5 and
 // 6-7 hold the low two bits, bits 20 and 21 the third.
@@ -116,8 +116,27 @@ __host__ __device__ constexpr int diag_class(int code) { return (code >> kDiagSh
 constexpr int kCodeAH = 1 << 19;
 // One-qubit matrix forms (read off the matrix on the host): general complex;
 // "RI" = real diagonal and imaginary off-diagonal (RX-like); real (RY-like);
-// diagonal (RZ / phase); the exact swap [[0,1],[1,0]] (X, the CNOT/Toffoli target).
-enum { kFormGen = 0, kFormRI = 1, kFormReal = 2, kFormDiag = 3, kFormSwap = 4 };
+// diagonal (RZ / phase); the exact swap [[0,1],[1,0]] (X, the CNOT/Toffoli
+// target).  The rest arise where the planner defers a gate's phases (fused.cu):
+// unit diagonal [[1,x],[y,1]], half the products of the general form; real
+// diagonal with a complex off-diagonal (a controlled rotation in a rotated
+// frame); off-diagonal (a controlled X); the identity (a diagonal gate deferred
+// whole).
+enum {
+  kFormGen = 0,
+  kFormRI = 1,
+  kFormReal = 2,
+  kFormDiag = 3,
+  kFormSwap = 4,
+  kFormUD = 5,
+  kFormRC = 6,
+  kFormOff = 7,
+  kFormId = 8,
+  kForms = 9
+};
+// Packed plan: the form's low three bits are code bits 11-13, the fourth bit 24.
+__host__ __device__ constexpr int form_of(int code) { return ((code >> 11) & 7) | (((code >> 24) & 1) << 3); }
+__host__ __device__ constexpr int form_bits(int form) { return ((form & 7) << 11) | ((form >> 3) << 24); }
 // Reduced-matrix entries a parameter's D touches: all four, off-diagonal,
 // diagonal; kAccAH added (FP32 body) when every D is anti-Hermitian and only
 // (Im A00, Im A11, Re A01 - Re A10, Im A01 + Im A10) are accumulated.

@@ -102,15 +102,17 @@ __host__ __device__ __forceinline__ uint32_t swz_pair(uint32_t p) {
 //   RI        p q -q s r -r   (u00 = p, u01 = i q, u10 = i r, u11 = s) (p,s) (-q,-r) (q,r)
 //   real      a00 a01 a10 a11                                      (a00,a11) (a01,a10)
 //   diagonal  d0r d0i -d0i d1r d1i -d1i                            (d0r,d1r) (d0i,d1i) (-d0i,-d1i)
-//   swap      (none)                                               (none)
-constexpr int kPoolFree[5] = {12, 6, 4, 6, 0};
-constexpr int kPoolLane[5] = {6, 3, 2, 3, 0};
+//   swap, identity (none)                                          (none)
+//   unit diag. xr xi -xi yr yi -yi  ([[1,x],[y,1]])                (xr,yr) (xi,yi) (-xi,-yi)
+//   real/cplx  a wr wi -wi d vr vi -vi  ([[a,w],[v,d]], a, d real) (a,d) (wr,vr) (wi,vi) (-wi,-vi)
+//   off-diag.  wr wi -wi vr vi -vi  ([[0,w],[v,0]])                (wr,vr) (wi,vi) (-wi,-vi)
 
 // Every free layout stores an imaginary part next to its negation, so conj(U)
 // (CJ: the reverse sweep holds the cotangent conjugated) is U with the two
 // exchanged: a compile-time permutation of the coefficient indices.
 template <bool CJ>
 struct FreeIx {
+  static constexpr int r2 = CJ ? 3 : 2, r3 = CJ ? 2 : 3, r6 = CJ ? 7 : 6, r7 = CJ ? 6 : 7;  // (real/complex)
   static constexpr int i1 = CJ ? 2 : 1, i2 = CJ ? 1 : 2, i4 = CJ ? 5 : 4, i5 = CJ ? 4 : 5, i7 = CJ ? 8 : 7,
                        i8 = CJ ? 7 : 8, i10 = CJ ? 11 : 10, i11 = CJ ? 10 : 11;
 };
@@ -140,7 +142,22 @@ __device__ __forceinline__ void free_apply(Pk& A, Pk& B, const u64* c) {
     A.i = fma2(c[0], ai, mul2(c[I::i1], ar));
     B.r = fma2(c[3], br, mul2(c[I::i5], bi));
     B.i = fma2(c[3], bi, mul2(c[I::i4], br));
-  } else {
+  } else if (FORM == kFormUD) {
+    A.r = fma2(c[0], br, fma2(c[I::i2], bi, ar));
+    A.i = fma2(c[0], bi, fma2(c[I::i1], br, ai));
+    B.r = fma2(c[3], ar, fma2(c[I::i5], ai, br));
+    B.i = fma2(c[3], ai, fma2(c[I::i4], ar, bi));
+  } else if (FORM == kFormRC) {
+    A.r = fma2(c[0], ar, fma2(c[1], br, mul2(c[I::r3], bi)));
+    A.i = fma2(c[0], ai, fma2(c[1], bi, mul2(c[I::r2], br)));
+    B.r = fma2(c[4], br, fma2(c[5], ar, mul2(c[I::r7], ai)));
+    B.i = fma2(c[4], bi, fma2(c[5], ai, mul2(c[I::r6], ar)));
+  } else if (FORM == kFormOff) {
+    A.r = fma2(c[0], br, mul2(c[I::i2], bi));
+    A.i = fma2(c[0], bi, mul2(c[I::i1], br));
+    B.r = fma2(c[3], ar, mul2(c[I::i5], ai));
+    B.i = fma2(c[3], ai, mul2(c[I::i4], ar));
+  } else if (FORM == kFormSwap) {
     const Pk t = A;
     A = B;
     B = t;
@@ -174,8 +191,25 @@ __device__ __forceinline__ void scalar_apply(Pk& A, Pk& B, const u64* c) {
     ai = fmaf(lo(c[0]), Ai, lo(c[I::i1]) * Ar);
     br = fmaf(lo(c[3]), Br, lo(c[I::i5]) * Bi);
     bi = fmaf(lo(c[3]), Bi, lo(c[I::i4]) * Br);
-  } else {
+  } else if (FORM == kFormUD) {
+    ar = fmaf(lo(c[0]), Br, fmaf(lo(c[I::i2]), Bi, Ar));
+    ai = fmaf(lo(c[0]), Bi, fmaf(lo(c[I::i1]), Br, Ai));
+    br = fmaf(lo(c[3]), Ar, fmaf(lo(c[I::i5]), Ai, Br));
+    bi = fmaf(lo(c[3]), Ai, fmaf(lo(c[I::i4]), Ar, Bi));
+  } else if (FORM == kFormRC) {
+    ar = fmaf(lo(c[0]), Ar, fmaf(lo(c[1]), Br, lo(c[I::r3]) * Bi));
+    ai = fmaf(lo(c[0]), Ai, fmaf(lo(c[1]), Bi, lo(c[I::r2]) * Br));
+    br = fmaf(lo(c[4]), Br, fmaf(lo(c[5]), Ar, lo(c[I::r7]) * Ai));
+    bi = fmaf(lo(c[4]), Bi, fmaf(lo(c[5]), Ai, lo(c[I::r6]) * Ar));
+  } else if (FORM == kFormOff) {
+    ar = fmaf(lo(c[0]), Br, lo(c[I::i2]) * Bi);
+    ai = fmaf(lo(c[0]), Bi, lo(c[I::i1]) * Br);
+    br = fmaf(lo(c[3]), Ar, lo(c[I::i5]) * Ai);
+    bi = fmaf(lo(c[3]), Ai, lo(c[I::i4]) * Ar);
+  } else if (FORM == kFormSwap) {
     ar = Br, ai = Bi, br = Ar, bi = Ai;
+  } else {
+    return;
   }
   if (LANE) {
     A.r = mk(lo(A.r), ar), A.i = mk(lo(A.i), ai), B.r = mk(lo(B.r), br), B.i = mk(lo(B.i), bi);
@@ -205,7 +239,22 @@ __device__ __forceinline__ void lane_apply(Pk& V, const u64* c) {
     constexpr int d1 = CJ ? 2 : 1, d2 = CJ ? 1 : 2;
     V.r = fma2(c[0], pr, mul2(c[d2], pi));
     V.i = fma2(c[0], pi, mul2(c[d1], pr));
-  } else {
+  } else if (FORM == kFormUD) {
+    constexpr int x1 = CJ ? 2 : 1, x2 = CJ ? 1 : 2;
+    const u64 qr = swp(pr), qi = swp(pi);
+    V.r = fma2(c[0], qr, fma2(c[x2], qi, pr));
+    V.i = fma2(c[0], qi, fma2(c[x1], qr, pi));
+  } else if (FORM == kFormRC) {
+    constexpr int x2 = CJ ? 3 : 2, x3 = CJ ? 2 : 3;
+    const u64 qr = swp(pr), qi = swp(pi);
+    V.r = fma2(c[0], pr, fma2(c[1], qr, mul2(c[x3], qi)));
+    V.i = fma2(c[0], pi, fma2(c[1], qi, mul2(c[x2], qr)));
+  } else if (FORM == kFormOff) {
+    constexpr int x1 = CJ ? 2 : 1, x2 = CJ ? 1 : 2;
+    const u64 qr = swp(pr), qi = swp(pi);
+    V.r = fma2(c[0], qr, mul2(c[x2], qi));
+    V.i = fma2(c[0], qi, mul2(c[x1], qr));
+  } else if (FORM == kFormSwap) {
     V.r = swp(pr);
     V.i = swp(pi);
   }
@@ -533,6 +582,10 @@ __device__ __forceinline__ void u1_form(int form, Pk (&v)[8], Pk (&w)[8], const 
     case kFormReal: u1_static<TB, CB, kFormReal, ADJ>(v, w, c); break;
     case kFormDiag: u1_static<TB, CB, kFormDiag, ADJ>(v, w, c); break;
     case kFormSwap: u1_static<TB, CB, kFormSwap, ADJ>(v, w, c); break;
+    case kFormUD: u1_static<TB, CB, kFormUD, ADJ>(v, w, c); break;
+    case kFormRC: u1_static<TB, CB, kFormRC, ADJ>(v, w, c); break;
+    case kFormOff: u1_static<TB, CB, kFormOff, ADJ>(v, w, c); break;
+    case kFormId: break;
     default: u1_static<TB, CB, kFormGen, ADJ>(v, w, c); break;
   }
 }
@@ -543,6 +596,10 @@ __device__ __forceinline__ void u1_form_masked(int form, Pk (&v)[8], Pk (&w)[8],
     case kFormReal: u1_masked<TB, kFormReal, ADJ>(v, w, c, rmask); break;
     case kFormDiag: u1_masked<TB, kFormDiag, ADJ>(v, w, c, rmask); break;
     case kFormSwap: u1_masked<TB, kFormSwap, ADJ>(v, w, c, rmask); break;
+    case kFormUD: u1_masked<TB, kFormUD, ADJ>(v, w, c, rmask); break;
+    case kFormRC: u1_masked<TB, kFormRC, ADJ>(v, w, c, rmask); break;
+    case kFormOff: u1_masked<TB, kFormOff, ADJ>(v, w, c, rmask); break;
+    case kFormId: break;
     default: u1_masked<TB, kFormGen, ADJ>(v, w, c, rmask); break;
   }
 }
@@ -1037,7 +1094,7 @@ __device__ __forceinline__ void interp_ops(const TileCtx<M, ADJ>& x, const DevSt
     if (!GEN || type == kOpU1) {
       const bool acc = ADJ && (code & kCodeAcc);
       if (!run && !acc) continue;
-      const int tb = (code >> 4) & 3, rctl = (code >> 16) & 7, form = (code >> 11) & 7, kind = acc_kind_of(code);
+      const int tb = (code >> 4) & 3, rctl = (code >> 16) & 7, form = form_of(code), kind = acc_kind_of(code);
       const uint32_t rmask = (uint32_t)op->rmask;
       float s8[8];
 #pragma unroll

@@ -14,7 +14,10 @@
 // Holding the 16 amplitudes in registers instead needs a variant per target
 // bit, and every switch then moves all of them between the variants' register
 // assignments: 1,360 instructions per op of a reverse FP64 pass, 395 of them
-// arithmetic (counted on 2^22 amplitudes), with the FP64 pipe at 25 %.
+// arithmetic (counted on 2^22 amplitudes), with the FP64 pipe at 25 %.  In
+// shared memory a 12-qubit FP64 reverse pass takes 73 us (93), a 17-qubit FP32
+// one 50 us (59), the serving loop's reverse launches 66 us (97); forward passes
+// are even (41, 31 and 57 us).
 #pragma once
 
 #include "engine.h"
@@ -197,6 +200,12 @@ __device__ __forceinline__ void tile_body(const TileItem& it) {
               case kFormReal: pair_acc<kFormReal, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
               case kFormDiag: pair_acc<kFormDiag, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
               case kFormSwap: pair_acc<kFormSwap, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
+              case kFormUD: pair_acc<kFormUD, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
+              case kFormRC: pair_acc<kFormRC, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
+              case kFormOff: pair_acc<kFormOff, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
+              case kFormId:
+                if (acc) pair_acc<kFormId, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T);
+                break;
               default: pair_acc<kFormGen, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
             }
           } else if (sel < kSelPhase) {

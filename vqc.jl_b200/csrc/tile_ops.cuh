@@ -48,7 +48,19 @@ __device__ __forceinline__ void u1_apply(C& x0, C& x1, const C (&u)[4]) {
   } else if (FORM == kFormDiag) {
     x0 = tmul(u[0], a);
     x1 = tmul(u[3], b);
-  } else {  // swap
+  } else if (FORM == kFormUD) {
+    x0 = tfma(u[1], b, a);
+    x1 = tfma(u[2], a, b);
+  } else if (FORM == kFormRC) {
+    const C t0 = tmul(u[1], b), t1 = tmul(u[2], a);
+    x0.x = fma(u[0].x, a.x, t0.x);
+    x0.y = fma(u[0].x, a.y, t0.y);
+    x1.x = fma(u[3].x, b.x, t1.x);
+    x1.y = fma(u[3].x, b.y, t1.y);
+  } else if (FORM == kFormOff) {
+    x0 = tmul(u[1], b);
+    x1 = tmul(u[2], a);
+  } else if (FORM == kFormSwap) {
     x0 = b;
     x1 = a;
   }

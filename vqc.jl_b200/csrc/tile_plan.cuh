@@ -36,6 +36,8 @@ struct FOp {
   Mat mat;               // U1 2x2, U2 4x4 (bit 0 <-> tq[0]), diagonal 2^nd table
   int nd = 0;
   int dq[5] = {0, 0, 0, 0, 0};
+  int form = -1;         // U1: a form chosen by its place (kForm*), -1: read off the matrix
+  double gain = 1;       // what executing the op multiplies the state's deferred norm by
   bool acc = false;
   std::vector<PGrad> grads;
 };
@@ -50,6 +52,7 @@ struct PassShape {
 struct AccRef {
   int row;
   std::vector<PGrad> grads;
+  double scale = 1;  // of the partials (the deferred norm squared when the op ran)
   bool ah = false;  // the row holds the anti-Hermitian projection (kAccAH)
 };
 
