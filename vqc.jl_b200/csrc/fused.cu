@@ -1037,7 +1037,7 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
         place_controls(o, cm, cv, tile_mask, tbit, st.rs, rc);
         int sel = k0 < 0 ? kSelDiag : (f.mat[k0] == cd(-1) ? kSelFlip : kSelPhase);
         if (f.kind == kOpU1) {
-          const int r = slot_of(tbit[f.tq[0]]), form = u1_form(f);
+          const int r = slot_of(tbit[f.tq[0]]), form = interpreted_form<R>(u1_form(f));
           sel = kSelU1 + (r | (rc.n ? 4 : 0) | form << 3);
           if (ADJ && f.acc) o.code |= (acc_kind(f) << 14) | (acc_anti_hermitian(f) ? kCodeAH : 0);
         }
@@ -1050,15 +1050,15 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
           for (int i = 0; i < (f.kind == kOpU1 ? 1 : 2); ++i) {
             const int r = slot_of(tbit[f.tq[i]]);
             held |= 1u << r;
-            o.target[i] = (uint16_t)s.swm[1 << r];
+            o.target[i] = (uint16_t)(s.swm[1 << r] * sizeof(cplx<R>));
           }
         for (auto& c : rc) {
           held |= 1u << c.first;
-          if (c.second) o.first ^= (uint16_t)s.swm[1 << c.first];
+          if (c.second) o.first ^= (uint16_t)(s.swm[1 << c.first] * sizeof(cplx<R>));
         }
         for (int r = 0; r < kRegBits; ++r)
           if (!(held >> r & 1)) {
-            if (nfree < 3) o.step[nfree] = (uint16_t)s.swm[1 << r];
+            if (nfree < 3) o.step[nfree] = (uint16_t)(s.swm[1 << r] * sizeof(cplx<R>));
             ++nfree;
           }
         o.code |= sel << kSelShift | nfree << 16;

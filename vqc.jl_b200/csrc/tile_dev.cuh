@@ -77,16 +77,17 @@ struct alignas(16) DevOp {
   int32_t code;
   int32_t mat;     // pool offset (complex elements)
   uint32_t cmask, cval;  // controls on tile bits
+  // classic body (second 16-byte word): the thread's amplitudes the op acts on,
+  // as byte offsets in the swizzled tile: first ^ (any combination of the
+  // op_free(code) entries of step), with the target bits at 0; target: what
+  // flips a target bit.  Both bodies: the accumulation slot, or -1.
+  uint16_t first, step[3], target[2];
+  int32_t slot;
   uint64_t gmask, gval;  // controls on non-tile qubits
-  int32_t slot;    // accumulation slot or -1
   int32_t nd;      // diagonal ops: number of qubits
   int32_t dbit[5];  // tile bit of diagonal qubit i, or -1
   int32_t dglob[5]; // global qubit of diagonal qubit i when not a tile bit
   int32_t rmask;    // register amplitudes (pair representatives) the controls enable
-  // classic body: the thread's amplitudes the op acts on, as swizzled tile
-  // indices: first ^ (any combination of the op_free(code) entries of step),
-  // with the target bits at 0; target: what flips a target bit
-  uint16_t first, step[3], target[2];
 };
 // The classic body's op variant (bits 24-30 of the code): one-qubit ops kSelU1
 // + (r0 | masked << 2 | form << 3), masked = a register control in rmask;

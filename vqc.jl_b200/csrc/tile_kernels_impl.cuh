@@ -15,9 +15,10 @@
 // bit, and every switch then moves all of them between the variants' register
 // assignments: 1,360 instructions per op of a reverse FP64 pass, 395 of them
 // arithmetic (counted on 2^22 amplitudes), with the FP64 pipe at 25 %.  In
-// shared memory a 12-qubit FP64 reverse pass takes 73 us (93), a 17-qubit FP32
-// one 50 us (59), the serving loop's reverse launches 66 us (97); forward passes
-// are even (41, 31 and 57 us).
+// shared memory a 12-qubit FP64 reverse pass takes 66 us (93), a 17-qubit FP32
+// one 46 us (59), the serving loop's reverse launches 68 us (97), a 17-qubit FP32
+// forward pass 28 us (31).  Bound by latency: a tile's few warps, each op's
+// decoding, loads and chain of FMAs one after another.
 #pragma once
 
 #include "engine.h"
@@ -29,22 +30,38 @@
 namespace vqc {
 
 // ----------------------------------------------------------------------------- ops in shared memory
-constexpr int kAccNone = 8;  // (after the kinds of kAcc*)
+constexpr int kAccNone = 3;  // (between the kinds of kAcc*: 0-2, 4-6)
 
-// N pairs, at a ^ off[i] and the same ^ t: all loads first (a pair's chain of
-// dependent FMAs is longer than a load, and a store bars the next load from
-// moving up), U on psi and lambda, the pairs' terms of the reduced matrix in
-// order, all stores.
+// The second 16-byte word of an op (DevOp: first, step, target, slot).
+struct OpWord {
+  uint32_t first, step[3], target[2];
+  int slot;
+  __device__ __forceinline__ explicit OpWord(int4 w) {
+    first = (uint32_t)w.x & 0xffffu, step[0] = (uint32_t)w.x >> 16;
+    step[1] = (uint32_t)w.y & 0xffffu, step[2] = (uint32_t)w.y >> 16;
+    target[0] = (uint32_t)w.z & 0xffffu, target[1] = (uint32_t)w.z >> 16;
+    slot = w.w;
+  }
+};
+template <class C>
+__device__ __forceinline__ C& at(unsigned char* tile, uint32_t byte) {
+  return *reinterpret_cast<C*>(tile + byte);
+}
+
+// N pairs, at a ^ off[i] and the same ^ t (bytes): all loads first (a pair's
+// chain of dependent FMAs is longer than a load, and a store bars the next load
+// from moving up), U on psi and lambda, the pairs' terms of the reduced matrix
+// in order, all stores.
 template <int N, int FORM, int ACC, bool ADJ, class R>
-__device__ __forceinline__ void pair_group(cplx<R>* sp, cplx<R>* sl, uint32_t a, uint32_t t, const uint32_t (&off)[4],
-                                           const cplx<R> (&u)[4], R (&acc)[8]) {
+__device__ __forceinline__ void pair_group(unsigned char* sp, unsigned char* sl, uint32_t a, uint32_t t,
+                                           const uint32_t (&off)[4], const cplx<R> (&u)[4], R (&acc)[8]) {
   using C = cplx<R>;
   C p0[N], p1[N], l0[N], l1[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const uint32_t b = a ^ off[i];
-    p0[i] = sp[b], p1[i] = sp[b ^ t];
-    if (ADJ) l0[i] = sl[b], l1[i] = sl[b ^ t];
+    const uint32_t b = a ^ off[i], c = b ^ t;
+    p0[i] = at<C>(sp, b), p1[i] = at<C>(sp, c);
+    if (ADJ) l0[i] = at<C>(sl, b), l1[i] = at<C>(sl, c);
   }
 #pragma unroll
   for (int i = 0; i < N; ++i) {
@@ -56,55 +73,70 @@ __device__ __forceinline__ void pair_group(cplx<R>* sp, cplx<R>* sl, uint32_t a,
   }
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const uint32_t b = a ^ off[i];
-    sp[b] = p0[i], sp[b ^ t] = p1[i];
-    if (ADJ) sl[b] = l0[i], sl[b ^ t] = l1[i];
+    const uint32_t b = a ^ off[i], c = b ^ t;
+    at<C>(sp, b) = p0[i], at<C>(sp, c) = p1[i];
+    if (ADJ) at<C>(sl, b) = l0[i], at<C>(sl, c) = l1[i];
   }
 }
 
 // The op's pairs in ascending order of their free bits (the compiled passes
 // sum in the same order), four at a time where there are four.
 template <int FORM, int ACC, bool ADJ, class R>
-__device__ __forceinline__ void pair_loop(cplx<R>* sp, cplx<R>* sl, uint32_t a, const DevOp* op, int nfree,
-                                          const cplx<R>* U, R (&acc)[8], [[maybe_unused]] int T) {
+__device__ __forceinline__ void pair_loop(unsigned char* sp, unsigned char* sl, uint32_t a, const OpWord& op,
+                                          int nfree, const cplx<R>* U, R (&acc)[8]) {
   const cplx<R> u[4] = {U[0], U[1], U[2], U[3]};
-  const uint32_t t = op->target[0], f0 = op->step[0], f1 = op->step[1];
-  const uint32_t off[4] = {0u, f0, f1, f0 ^ f1};
-  if (!VQC_DCHECK(a ^ t, T)) return;
+  const uint32_t t = op.target[0], off[4] = {0u, op.step[0], op.step[1], op.step[0] ^ op.step[1]};
   if (nfree >= 2) {
     pair_group<4, FORM, ACC, ADJ, R>(sp, sl, a, t, off, u, acc);
-    if (nfree == 3) pair_group<4, FORM, ACC, ADJ, R>(sp, sl, a ^ op->step[2], t, off, u, acc);
+    if (nfree == 3) pair_group<4, FORM, ACC, ADJ, R>(sp, sl, a ^ op.step[2], t, off, u, acc);
   } else {
     pair_group<1, FORM, ACC, ADJ, R>(sp, sl, a, t, off, u, acc);
-    if (nfree == 1) pair_group<1, FORM, ACC, ADJ, R>(sp, sl, a ^ f0, t, off, u, acc);
+    if (nfree == 1) pair_group<1, FORM, ACC, ADJ, R>(sp, sl, a ^ off[1], t, off, u, acc);
   }
 }
-template <int FORM, bool ADJ, class R>
-__device__ __forceinline__ void pair_acc(int acck, cplx<R>* sp, cplx<R>* sl, uint32_t a, const DevOp* op, int nfree,
-                                         const cplx<R>* U, R (&acc)[8], int T) {
+
+// One switch over the matrix form and what the op sums of the reduced matrix.
+template <bool ADJ, class R>
+__device__ __forceinline__ void pair_switch(int form, int acck, unsigned char* sp, unsigned char* sl, uint32_t a,
+                                            const OpWord& op, int nfree, const cplx<R>* U, R (&acc)[8]) {
+#define VQC_FORMS(X, K)                                                                                        \
+  X(kFormGen, K) X(kFormRI, K) X(kFormReal, K) X(kFormDiag, K) X(kFormSwap, K) X(kFormUD, K) X(kFormRC, K) \
+  X(kFormOff, K) X(kFormId, K)
+#define VQC_CASE(F, K)                                                                          \
+  case F + kForms * K:                                                                          \
+    if constexpr (interpreted_form<R>(F) == F) pair_loop<F, K, ADJ, R>(sp, sl, a, op, nfree, U, acc); \
+    break;
   if constexpr (ADJ) {
-    switch (acck) {
-      case kAccFull: pair_loop<FORM, kAccFull, ADJ, R>(sp, sl, a, op, nfree, U, acc, T); return;
-      case kAccOff: pair_loop<FORM, kAccOff, ADJ, R>(sp, sl, a, op, nfree, U, acc, T); return;
-      case kAccDiag: pair_loop<FORM, kAccDiag, ADJ, R>(sp, sl, a, op, nfree, U, acc, T); return;
-      case kAccAH | kAccFull: pair_loop<FORM, kAccAH | kAccFull, ADJ, R>(sp, sl, a, op, nfree, U, acc, T); return;
-      case kAccAH | kAccOff: pair_loop<FORM, kAccAH | kAccOff, ADJ, R>(sp, sl, a, op, nfree, U, acc, T); return;
-      case kAccAH | kAccDiag: pair_loop<FORM, kAccAH | kAccDiag, ADJ, R>(sp, sl, a, op, nfree, U, acc, T); return;
+    switch (form + kForms * acck) {
+      VQC_FORMS(VQC_CASE, kAccFull)
+      VQC_FORMS(VQC_CASE, kAccOff)
+      VQC_FORMS(VQC_CASE, kAccDiag)
+      VQC_FORMS(VQC_CASE, (kAccAH | kAccFull))
+      VQC_FORMS(VQC_CASE, (kAccAH | kAccOff))
+      VQC_FORMS(VQC_CASE, (kAccAH | kAccDiag))
+      VQC_FORMS(VQC_CASE, kAccNone)
+      default: break;
+    }
+  } else {
+    switch (form + kForms * kAccNone) {
+      VQC_FORMS(VQC_CASE, kAccNone)
       default: break;
     }
   }
-  pair_loop<FORM, kAccNone, ADJ, R>(sp, sl, a, op, nfree, U, acc, T);
+#undef VQC_CASE
+#undef VQC_FORMS
 }
 
 template <class R>
-__device__ __forceinline__ void quad_loop(cplx<R>* s, uint32_t a, const DevOp* op, int nfree, const cplx<R>* U) {
+__device__ __forceinline__ void quad_loop(unsigned char* s, uint32_t a, const OpWord& op, int nfree,
+                                          const cplx<R>* U) {
   using C = cplx<R>;
-  const uint32_t ta = op->target[0], tb = op->target[1];
+  const uint32_t ta = op.target[0], tb = op.target[1];
   for (int k = 0; k < (1 << nfree); ++k) {
-    const uint32_t b = a ^ ((k & 1) ? op->step[0] : 0u) ^ ((k & 2) ? op->step[1] : 0u);
-    C x0 = s[b], x1 = s[b ^ ta], x2 = s[b ^ tb], x3 = s[b ^ ta ^ tb];
+    const uint32_t b = a ^ ((k & 1) ? op.step[0] : 0u) ^ ((k & 2) ? op.step[1] : 0u);
+    C x0 = at<C>(s, b), x1 = at<C>(s, b ^ ta), x2 = at<C>(s, b ^ tb), x3 = at<C>(s, b ^ ta ^ tb);
     u2_quad(x0, x1, x2, x3, U);
-    s[b] = x0, s[b ^ ta] = x1, s[b ^ tb] = x2, s[b ^ ta ^ tb] = x3;
+    at<C>(s, b) = x0, at<C>(s, b ^ ta) = x1, at<C>(s, b ^ tb) = x2, at<C>(s, b ^ ta ^ tb) = x3;
   }
 }
 
@@ -154,10 +186,13 @@ __device__ __forceinline__ void tile_body(const TileItem& it) {
   const int nstages = it.p.stage_end - it.p.stage_begin;
   C* sp = x.sp;
   C* sl = x.sl;
+  unsigned char* bp = reinterpret_cast<unsigned char*>(sp);
+  unsigned char* bl = reinterpret_cast<unsigned char*>(sl);
   for (int64_t tile = blockIdx.x; tile < it.p.ntiles; tile += it.ncta) {
     for (int s = 0; s < nstages; ++s) {
       const DevStage* S = x.stages + s;
       const uint32_t tthr = S->thr[0][x.tlo] | S->thr[1][x.thi], sw = S->swt[0][x.tlo] ^ S->swt[1][x.thi];
+      const uint32_t swb = sw * (uint32_t)sizeof(C);
       if (s == 0) {
         C v[16], w[16];
         tile_load<R, ADJ>(x, S, true, v, w, S->swm, S->gdep);
@@ -170,13 +205,17 @@ __device__ __forceinline__ void tile_body(const TileItem& it) {
         }
       }
       const int oe = S->op_end;
-      int o = S->op_begin;
-      int4 hd = o < oe ? *reinterpret_cast<const int4*>(x.ops + o) : make_int4(0, 0, 0, 0);
+      int o = S->op_begin, held = -1;  // held: the slot of an op whose sums wait for a second op's
+      R ha[4];
+      const int4* words = reinterpret_cast<const int4*>(x.ops + o);
+      int4 w0 = words[0], w1 = words[1];  // (read one op ahead; the word after the last op is in the tables)
 #pragma unroll 1
       for (; o < oe; ++o) {
         const DevOp* op = x.ops + o;
-        const int4 cur = hd;
-        if (o + 1 < oe) hd = *reinterpret_cast<const int4*>(op + 1);
+        const int4 cur = w0;
+        const OpWord ow(w1);
+        words += sizeof(DevOp) / 16;
+        if (o + 1 < oe) w0 = words[0], w1 = words[1];
         const int code = cur.x, sel = (code >> kSelShift) & 127;
         if (code & kCodeGCtl) {  // a control on a non-tile qubit: uniform over the tile
           if ((x.base & op->gmask) != op->gval) continue;
@@ -186,31 +225,20 @@ __device__ __forceinline__ void tile_body(const TileItem& it) {
         const bool run = !(code & kCodeCtl) || (tthr & (uint32_t)cur.z) == (uint32_t)cur.w;
         const bool acc = ADJ && (code & kCodeAcc);
         const C* U = x.pool + cur.y;
-        const int kind = acc_kind_of(code), acck = acc ? kind : kAccNone, nf = op_free(code);
+        const int kind = acc_kind_of(code), nf = op_free(code);
         R a[8];
         if (ADJ) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) a[i] = R(0);
         }
         if (run) {
-          const uint32_t t = sw ^ op->first;
+          const uint32_t t = swb ^ ow.first;
           if (sel < kSelU2) {
-            switch (sel >> 3) {
-              case kFormRI: pair_acc<kFormRI, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
-              case kFormReal: pair_acc<kFormReal, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
-              case kFormDiag: pair_acc<kFormDiag, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
-              case kFormSwap: pair_acc<kFormSwap, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
-              case kFormUD: pair_acc<kFormUD, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
-              case kFormRC: pair_acc<kFormRC, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
-              case kFormOff: pair_acc<kFormOff, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
-              case kFormId:
-                if (acc) pair_acc<kFormId, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T);
-                break;
-              default: pair_acc<kFormGen, ADJ, R>(acck, sp, sl, t, op, nf, U, a, x.T); break;
-            }
+            if (VQC_DCHECK(t ^ ow.target[0], sizeof(C) * x.T))
+              pair_switch<ADJ, R>(sel >> 3, acc ? kind : kAccNone, bp, bl, t, ow, nf, U, a);
           } else if (sel < kSelPhase) {
-            quad_loop<R>(sp, t, op, nf, U);
-            if (ADJ) quad_loop<R>(sl, t, op, nf, U);
+            quad_loop<R>(bp, t, ow, nf, U);
+            if (ADJ) quad_loop<R>(bl, t, ow, nf, U);
           } else if (sel == kSelFlip) {
             phase_loop<true, R>(sp, sw, S, (uint32_t)op->rmask, U);
             if (ADJ) phase_loop<true, R>(sl, sw, S, (uint32_t)op->rmask, U);
@@ -224,11 +252,21 @@ __device__ __forceinline__ void tile_body(const TileItem& it) {
           }
         }
         if (acc) {
-          if (kind & kAccAH)
-            flush_acc<4>(a, tile_slot(x, op->slot));
-          else
-            flush_acc<8>(a, tile_slot(x, op->slot));
+          if (!(kind & kAccAH)) {
+            flush_acc<8>(a, tile_slot(x, ow.slot));
+          } else if (held < 0) {
+            held = ow.slot;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ha[i] = a[i];
+          } else {
+            flush_two(ha, a, tile_slot(x, held), tile_slot(x, ow.slot));
+            held = -1;
+          }
         }
+      }
+      if (ADJ && held >= 0) {
+        R a[8] = {ha[0], ha[1], ha[2], ha[3], R(0), R(0), R(0), R(0)};
+        flush_acc<4>(a, tile_slot(x, held));
       }
       if (s == nstages - 1) {
         C v[16], w[16];
@@ -251,11 +289,12 @@ __device__ __forceinline__ void tile_body(const TileItem& it) {
   tile_end(x, it);
 }
 
-// Resident CTAs: what the tiles in shared memory admit (32 KiB, reverse 64 KiB,
-// plus descriptors), registers budgeted for it.
+// Resident CTAs the registers are budgeted for: forward what the tiles in shared
+// memory admit (32 KiB each plus descriptors); reverse two, without spills (at
+// three a 17-qubit FP32 reverse pass takes 70 against 46 us).
 template <class R, bool ADJ>
 struct TileBounds {
-  static constexpr int nt = sizeof(R) == 4 ? 256 : 128, nb = ADJ ? 3 : 5;
+  static constexpr int nt = sizeof(R) == 4 ? 256 : 128, nb = ADJ ? 2 : 5;
 };
 
 template <class R, bool ADJ>

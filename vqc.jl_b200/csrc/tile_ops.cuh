@@ -17,7 +17,7 @@ template <class C>
 __device__ __forceinline__ C tmul(C a, C b) {
   C r;
   r.x = fma(a.x, b.x, -a.y * b.y);
-  r.y = fma(a.x, b.y, a.y * b.x);
+  r.y = fma(a.y, b.x, a.x * b.y);
   return r;
 }
 template <class C>
@@ -29,6 +29,8 @@ __device__ __forceinline__ C tfma(C a, C b, C acc) {
   return acc;
 }
 
+// U on one pair.  The structured forms round like the general one (a product
+// with an exact zero left out), so that a gate's bits do not depend on its form.
 template <int FORM, class C>
 __device__ __forceinline__ void u1_apply(C& x0, C& x1, const C (&u)[4]) {
   const C a = x0, b = x1;
@@ -36,18 +38,19 @@ __device__ __forceinline__ void u1_apply(C& x0, C& x1, const C (&u)[4]) {
     x0 = tfma(u[1], b, tmul(u[0], a));
     x1 = tfma(u[3], b, tmul(u[2], a));
   } else if (FORM == kFormRI) {  // u00 = p, u01 = i q, u10 = i r, u11 = s (p, q, r, s real)
-    x0.x = fma(u[0].x, a.x, -u[1].y * b.y);
-    x0.y = fma(u[0].x, a.y, u[1].y * b.x);
+    x0.x = fma(-u[1].y, b.y, u[0].x * a.x);
+    x0.y = fma(u[1].y, b.x, u[0].x * a.y);
     x1.x = fma(u[3].x, b.x, -u[2].y * a.y);
     x1.y = fma(u[3].x, b.y, u[2].y * a.x);
   } else if (FORM == kFormReal) {
-    x0.x = fma(u[0].x, a.x, u[1].x * b.x);
-    x0.y = fma(u[0].x, a.y, u[1].x * b.y);
-    x1.x = fma(u[2].x, a.x, u[3].x * b.x);
-    x1.y = fma(u[2].x, a.y, u[3].x * b.y);
+    x0.x = fma(u[1].x, b.x, u[0].x * a.x);
+    x0.y = fma(u[1].x, b.y, u[0].x * a.y);
+    x1.x = fma(u[3].x, b.x, u[2].x * a.x);
+    x1.y = fma(u[3].x, b.y, u[2].x * a.y);
   } else if (FORM == kFormDiag) {
     x0 = tmul(u[0], a);
-    x1 = tmul(u[3], b);
+    x1.x = fma(-u[3].y, b.y, u[3].x * b.x);
+    x1.y = fma(u[3].y, b.x, u[3].x * b.y);
   } else if (FORM == kFormUD) {
     x0 = tfma(u[1], b, a);
     x1 = tfma(u[2], a, b);
@@ -220,10 +223,10 @@ __device__ __forceinline__ void op_acc(const cplx<R> (&v)[16], const cplx<R> (&w
   }
 }
 
-// Thread partials -> the warp's slot row: a warp reduce-scatter in FP64 of the
-// first N (4 or 8) values; every lane of the warp must call it.
+// A warp reduce-scatter in FP64 of the first N (4 or 8) values: lane
+// i * (32 / N) ends with the total of value i.  Every lane must call it.
 template <int N, class R>
-__device__ __forceinline__ void flush_acc(const R (&a)[8], double* row) {
+__device__ __forceinline__ double warp_scatter(const R (&a)[8]) {
   const int lane = threadIdx.x & 31;
   double x[N];
 #pragma unroll
@@ -240,7 +243,23 @@ __device__ __forceinline__ void flush_acc(const R (&a)[8], double* row) {
   }
 #pragma unroll
   for (; o > 0; o >>= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
-  if ((lane & (32 / N - 1)) == 0) row[lane / (32 / N)] += x[0];
+  return x[0];
+}
+// Thread partials -> the warp's slot row.
+template <int N, class R>
+__device__ __forceinline__ void flush_acc(const R (&a)[8], double* row) {
+  const double u = warp_scatter<N>(a);
+  const int lane = threadIdx.x & 31;
+  if ((lane & (32 / N - 1)) == 0) row[lane / (32 / N)] += u;
+}
+// Two ops' first four values at once: nine exchanges instead of twelve and one
+// chain of them instead of two; every value's sum has the same order.
+template <class R>
+__device__ __forceinline__ void flush_two(const R (&a)[4], const R (&b)[8], double* rowa, double* rowb) {
+  const R both[8] = {a[0], a[1], a[2], a[3], b[0], b[1], b[2], b[3]};
+  const double u = warp_scatter<8>(both);
+  const int lane = threadIdx.x & 31, i = lane >> 2;
+  if ((lane & 3) == 0) (i < 4 ? rowa : rowb - 4)[i] += u;
 }
 
 // ----------------------------------------------------------------------------- a pass

@@ -23,6 +23,14 @@ struct Swz<double> {  // 16-byte amplitudes: quarter-warps must hit 8 distinct 1
   __host__ __device__ static __forceinline__ uint32_t f(uint32_t t) { return t ^ (((t >> 3) ^ (t >> 6)) & 7u); }
 };
 
+// The form the classic body runs a one-qubit op in.  The forms of deferred
+// phases come to it in FP64 only (a compiled circuit's first call); the FP32
+// body leaves them out, its registers and instruction cache are the smaller for it.
+template <class R>
+__host__ __device__ constexpr int interpreted_form(int form) {
+  return sizeof(R) == 4 && form > kFormSwap ? (int)kFormGen : form;
+}
+
 struct PGrad {
   int param;             // caller's parameter index
   Mat2 D;                // U1: 2x2 over the target (control subspace); AccD: 2^nd diagonal bins
