@@ -125,7 +125,10 @@ __global__ void __launch_bounds__(kRedThreads) k_dm_trace(const cplx<R>* __restr
 // multiplication), op = identity or the conjugate transpose.  Work item =
 // (column j, row group r0 with the K target bits clear):
 //   (M B)[r_s][j] = sum_t M[s][t] B[r_t][j],  sum_s A[j][r_s] (M B)[r_s][j].
-// FP64 accumulation and grid reduction.
+// FP64 accumulation and grid reduction.  Consecutive threads take consecutive
+// row groups, or consecutive columns (COLS) where both matrices are read across
+// (op(A) = A, op(B) = B^dagger: entries j + N r, adjacent in j): across rows
+// those two reads touched a sector per entry.
 template <int K>
 struct TraceProdArgs {
   double2 M[(1 << K) * (1 << K)];  // sorted-position order, row-major
@@ -133,7 +136,7 @@ struct TraceProdArgs {
   int sp[K];                       // sorted target bits
 };
 
-template <class R, int K>
+template <class R, int K, bool COLS>
 __global__ void __launch_bounds__(kRedThreads)
     k_dm_trace_prod(const cplx<R>* __restrict__ a, const cplx<R>* __restrict__ b, int n, int dag_a, int dag_b,
                     const __grid_constant__ TraceProdArgs<K> g, Scratch s, double* res) {
@@ -141,8 +144,8 @@ __global__ void __launch_bounds__(kRedThreads)
   const int64_t N = int64_t(1) << n, rows = N >> K, items = rows << n;
   double acc[2] = {0, 0};
   for (int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; it < items; it += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = it >> (n - K);
-    int64_t r0 = it & (rows - 1);
+    const int64_t j = COLS ? it & (N - 1) : it >> (n - K);
+    int64_t r0 = COLS ? it >> n : it & (rows - 1);
 #pragma unroll
     for (int q = 0; q < K; ++q) r0 = ((r0 >> g.sp[q]) << (g.sp[q] + 1)) | (r0 & ((int64_t(1) << g.sp[q]) - 1));
     double2 bv[D];
@@ -181,12 +184,16 @@ static int trace_prod_k(vqc_state a, vqc_state b, int dag_a, int dag_b, const in
   const int n = b->n_dm;
   const int grid = reduction_grid(b->device, (int64_t(1) << (2 * n - K)));
   ProfScope prof(b->stream, "dm_trace_prod", 2.0 * (double)b->size() * b->amp_bytes());
-  if (b->dtype == VQC_C64)
-    k_dm_trace_prod<float, K><<<grid, kRedThreads, 0, b->stream>>>((const float2*)a->d, (const float2*)b->d, n, dag_a,
-                                                                    dag_b, g, b->scr, b->scr.result);
-  else
-    k_dm_trace_prod<double, K><<<grid, kRedThreads, 0, b->stream>>>((const double2*)a->d, (const double2*)b->d, n,
-                                                                     dag_a, dag_b, g, b->scr, b->scr.result);
+  const bool cols = !dag_a && dag_b;
+  if (b->dtype == VQC_C64) {
+    auto k = cols ? k_dm_trace_prod<float, K, true> : k_dm_trace_prod<float, K, false>;
+    k<<<grid, kRedThreads, 0, b->stream>>>((const float2*)a->d, (const float2*)b->d, n, dag_a, dag_b, g, b->scr,
+                                           b->scr.result);
+  } else {
+    auto k = cols ? k_dm_trace_prod<double, K, true> : k_dm_trace_prod<double, K, false>;
+    k<<<grid, kRedThreads, 0, b->stream>>>((const double2*)a->d, (const double2*)b->d, n, dag_a, dag_b, g, b->scr,
+                                           b->scr.result);
+  }
   VQC_CK(cudaGetLastError());
   int rc = fetch_result(b, 2);
   if (rc) return rc;
