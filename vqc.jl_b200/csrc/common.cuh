@@ -145,6 +145,8 @@ struct vqc_state_s {
   size_t accbuf_rows = 0;
   void* fused_scratch = nullptr;  // per-CTA partial sums of the tile engine
   size_t fused_scratch_bytes = 0;
+  void* outbuf = nullptr;  // results on their way to the host (partial trace, probabilities)
+  size_t outbuf_bytes = 0;
   std::mutex mu;
   size_t amp_bytes() const { return dtype == VQC_C64 ? 8 : 16; }
   int64_t size() const { return int64_t(1) << nq; }
@@ -161,6 +163,11 @@ int stream_after(vqc_state dst, vqc_state src);
 int workspace(vqc_state h, int count, void** bufs);
 // Makes h's device current; returns a status.
 int enter(vqc_state h);
+// Device memory of handles.  dev_free keeps buffers for later handles (at most
+// kPoolBytes per device; all are given back when the device's last handle goes
+// or an allocation fails); every use of a buffer must have completed.
+int dev_alloc(int device, void** p, size_t bytes);
+void dev_free(int device, void* p, size_t bytes);
 // Grows h->opbuf to at least `bytes` and copies `src` into it (stream-ordered).
 int upload_ops(vqc_state h, const void* src, size_t bytes);
 int reserve_ops(vqc_state h, size_t bytes);

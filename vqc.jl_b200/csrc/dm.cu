@@ -58,6 +58,23 @@ int dm_apply_gate_raw(vqc_state h, int k, const int* pos, const double* mat) {
   return apply_gate_raw(h, k, p2, Uc.data());
 }
 
+// The handle's buffer of results for the host, kept between calls: a
+// stream-ordered allocation per call gave its memory back to the driver at every
+// synchronisation (12 qubits: partial trace 1.87 -> 0.84 ms, probabilities 576 ->
+// 35 us).
+static int reserve_out(vqc_state h, size_t bytes) {
+  if (bytes <= h->outbuf_bytes) return VQC_OK;
+  if (h->outbuf) {
+    VQC_CK(cudaStreamSynchronize(h->stream));
+    VQC_CK(cudaFree(h->outbuf));
+    h->outbuf = nullptr;
+    h->outbuf_bytes = 0;
+  }
+  if (int rc = dev_alloc(h->device, &h->outbuf, bytes)) return rc;
+  h->outbuf_bytes = bytes;
+  return VQC_OK;
+}
+
 // rho[r + L c] = psi[r] conj(psi[c])
 template <class R>
 __global__ void k_dm_from_state(cplx<R>* rho, const cplx<R>* psi, int n) {
@@ -362,8 +379,8 @@ int vqc_dm_ptrace(vqc_state rho, int nsites, const int* sites, double* out) {
   const int nk = n - nsites;
   const int64_t s1 = int64_t(1) << nk;
   std::lock_guard<std::mutex> lk(rho->mu);
-  double2* dout = nullptr;
-  VQC_CK(cudaMallocAsync((void**)&dout, sizeof(double2) * s1 * s1, rho->stream));
+  if ((rc = reserve_out(rho, sizeof(double2) * s1 * s1))) return rc;
+  double2* dout = (double2*)rho->outbuf;
   const int g = launch_grid(rho->device, s1 * s1);
   if (rho->dtype == VQC_C64)
     k_dm_ptrace<float><<<g, 256, 0, rho->stream>>>((const float2*)rho->d, n, kept, traced, nk, nsites, dout);
@@ -372,7 +389,6 @@ int vqc_dm_ptrace(vqc_state rho, int nsites, const int* sites, double* out) {
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(out, dout, sizeof(double2) * s1 * s1, cudaMemcpyDeviceToHost, rho->stream);
-  cudaFreeAsync(dout, rho->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(rho->stream);
   if (e != cudaSuccess) return cuda_fail(e, "partial trace");
   return VQC_OK;
@@ -386,8 +402,8 @@ int vqc_dm_probs(vqc_state rho, double* out) {
   if (!out) return fail(VQC_ERR_ARG, "null output");
   std::lock_guard<std::mutex> lk(rho->mu);
   const int64_t L = int64_t(1) << n;
-  double* dout = nullptr;
-  VQC_CK(cudaMallocAsync((void**)&dout, sizeof(double) * L, rho->stream));
+  if ((rc = reserve_out(rho, sizeof(double) * L))) return rc;
+  double* dout = (double*)rho->outbuf;
   const int g = launch_grid(rho->device, L);
   if (rho->dtype == VQC_C64)
     k_dm_diag<float><<<g, 256, 0, rho->stream>>>((const float2*)rho->d, n, dout);
@@ -395,7 +411,6 @@ int vqc_dm_probs(vqc_state rho, double* out) {
     k_dm_diag<double><<<g, 256, 0, rho->stream>>>((const double2*)rho->d, n, dout);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(out, dout, sizeof(double) * L, cudaMemcpyDeviceToHost, rho->stream);
-  cudaFreeAsync(dout, rho->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(rho->stream);
   if (e != cudaSuccess) return cuda_fail(e, "probabilities");
   return VQC_OK;
