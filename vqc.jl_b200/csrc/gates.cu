@@ -92,23 +92,27 @@ int analyze_gate(int n, int k, const int* pos, const double* mat, bool dagger, G
   return VQC_OK;
 }
 
-template <class R, int MS, int MODE>
+// FULL: every index of the group is active (ns = MS), no tests in the product: a
+// dense two-qubit gate takes 690 instead of 770 to 830 us on 2^28 FP32 amplitudes
+// (three qubits 800 instead of 705: up to MS = 4 only).
+template <class R, int MS, int MODE, bool FULL>
 __global__ void __launch_bounds__(256) k_gate_sub(cplx<R>* __restrict__ v, const __grid_constant__ SubArgs<R, MS> a) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < a.ngroups; g += stride) {
     const int64_t base = group_base(g, a.k, a.mask);
     cplx<R> x[MS];
     if (MODE == kDense) {
+      const int ns = FULL ? MS : a.ns;
 #pragma unroll
       for (int s = 0; s < MS; ++s)
-        if (s < a.ns && VQC_DCHECK(base + a.off[s], a.namp)) x[s] = v[base + a.off[s]];
+        if (s < ns && VQC_DCHECK(base + a.off[s], a.namp)) x[s] = v[base + a.off[s]];
 #pragma unroll
       for (int r = 0; r < MS; ++r) {
-        if (r < a.ns) {
+        if (r < ns) {
           cplx<R> acc = mkc<R>(R(0), R(0));
 #pragma unroll
           for (int c = 0; c < MS; ++c)
-            if (c < a.ns) acc = cfma(a.U[r * MS + c], x[c], acc);
+            if (c < ns) acc = cfma(a.U[r * MS + c], x[c], acc);
           if (VQC_DCHECK(base + a.off[r], a.namp)) v[base + a.off[r]] = acc;
         }
       }
@@ -127,6 +131,57 @@ __global__ void __launch_bounds__(256) k_gate_sub(cplx<R>* __restrict__ v, const
   }
 }
 
+// Dense four- and five-qubit gates: MS x MS products per group of MS amplitudes
+// (16 and 32 complex FMAs per amplitude), bound by the FMA pipe.  The matrix sits
+// in shared memory and is read by broadcast; a thread keeps its group in registers
+// and forms one output row at a time, real and imaginary products in separate
+// chains.  k_gate_sub reads the matrix as kernel parameters: up to 16 KiB of them
+// stream through the constant cache for every group.  Measured at 2^28 FP32 / 2^26
+// FP64 amplitudes: five qubits 2.29 -> 1.88 ms / 1.70 -> 0.91 ms, four 1.04 -> 0.96
+// ms / 838 -> 457 us (FMA floor of five: 0.94 / 0.47 ms).  Two FP32 groups per thread
+// on packed FMAs: 2.93 ms (moves to pair the operands).
+template <class R>
+constexpr int kDensePerSm = sizeof(R) == 4 ? 4 : 3;  // resident CTAs (the grid: a larger one ends in a nearly empty wave)
+template <class R, int MS>
+__global__ void __launch_bounds__(128, kDensePerSm<R>)
+    k_gate_dense(cplx<R>* __restrict__ v, const __grid_constant__ SubArgs<R, MS> a) {
+  using C = cplx<R>;
+  __shared__ __align__(16) C U[MS * MS];
+  __shared__ int64_t off[MS];
+  for (int i = threadIdx.x; i < MS * MS; i += 128) U[i] = a.U[i];
+  if (threadIdx.x < MS) off[threadIdx.x] = a.off[threadIdx.x];
+  __syncthreads();
+  const int64_t step = (int64_t)gridDim.x * 128;
+  for (int64_t g = blockIdx.x * (int64_t)128 + threadIdx.x; g < a.ngroups; g += step) {
+    const int64_t base = group_base(g, a.k, a.mask);
+    C x[MS];
+#pragma unroll
+    for (int c = 0; c < MS; ++c)
+      if (VQC_DCHECK(base + off[c], a.namp)) x[c] = v[base + off[c]];
+#pragma unroll 1
+    for (int r = 0; r < MS; ++r) {
+      R rr = 0, ii = 0, ri = 0, ir = 0;
+#pragma unroll
+      for (int c = 0; c < MS; ++c) {
+        const C u = U[r * MS + c];
+        rr = fma(u.x, x[c].x, rr);
+        ii = fma(u.y, x[c].y, ii);
+        ri = fma(u.x, x[c].y, ri);
+        ir = fma(u.y, x[c].x, ir);
+      }
+      if (VQC_DCHECK(base + off[r], a.namp)) v[base + off[r]] = mkc<R>(rr - ii, ri + ir);
+    }
+  }
+}
+
+template <class R, int MS>
+static int launch_dense(const SubArgs<R, MS>& a, void* v, int device, cudaStream_t stream) {
+  const int grid = (int)std::min<int64_t>((a.ngroups + 127) / 128, (int64_t)device_info(device).sms * kDensePerSm<R>);
+  k_gate_dense<R, MS><<<grid, 128, 0, stream>>>((cplx<R>*)v, a);
+  VQC_CK(cudaGetLastError());
+  return VQC_OK;
+}
+
 template <class R, int MS>
 static int launch_ms(const GateSpec& g, void* v, int nq, int device, cudaStream_t stream) {
   SubArgs<R, MS> a;
@@ -134,12 +189,24 @@ static int launch_ms(const GateSpec& g, void* v, int nq, int device, cudaStream_
   const int grid = launch_grid(device, a.ngroups);
   ProfScope prof(stream, g.mode == kDense ? "gate_dense" : (g.mode == kDiag ? "gate_diag" : "gate_perm"),
                  2.0 * a.ngroups * g.ns * sizeof(cplx<R>));
+  if constexpr (MS <= 4) {
+    if (g.mode == kDense && g.ns == MS) {
+      k_gate_sub<R, MS, kDense, true><<<grid, 256, 0, stream>>>((cplx<R>*)v, a);
+      VQC_CK(cudaGetLastError());
+      return VQC_OK;
+    }
+  }
+  if constexpr (MS >= 16) {
+    // (the four lowest qubits: a thread's amplitudes are one run, and k_gate_sub's
+    // fewer registers win)
+    if (g.mode == kDense && g.ns == MS && (MS == 32 || g.sp[3] > 3)) return launch_dense<R, MS>(a, v, device, stream);
+  }
   if (g.mode == kDense)
-    k_gate_sub<R, MS, kDense><<<grid, 256, 0, stream>>>((cplx<R>*)v, a);
+    k_gate_sub<R, MS, kDense, false><<<grid, 256, 0, stream>>>((cplx<R>*)v, a);
   else if (g.mode == kDiag)
-    k_gate_sub<R, MS, kDiag><<<grid, 256, 0, stream>>>((cplx<R>*)v, a);
+    k_gate_sub<R, MS, kDiag, false><<<grid, 256, 0, stream>>>((cplx<R>*)v, a);
   else
-    k_gate_sub<R, MS, kMono><<<grid, 256, 0, stream>>>((cplx<R>*)v, a);
+    k_gate_sub<R, MS, kMono, false><<<grid, 256, 0, stream>>>((cplx<R>*)v, a);
   VQC_CK(cudaGetLastError());
   return VQC_OK;
 }
