@@ -2,10 +2,9 @@
 
 Both run the same device functions in the same order, so a state, an energy
 and a gradient have the same bits whichever kernel ran: a circuit's first call
-(interpreted, while its passes compile in the background) and its later ones
-agree exactly.  The oracle bounds of both are asserted elsewhere
-(test_gpu_fused.py, test_gpu_tile_forms.py, test_gpu_diag_ops.py with VQC_JIT on
-and off).
+(interpreted) and its later ones (compiled, from the second on) agree exactly.
+The oracle bounds of both are asserted elsewhere (test_gpu_fused.py,
+test_gpu_tile_forms.py, test_gpu_diag_ops.py with VQC_JIT on and off).
 """
 import numpy as np
 import pytest

@@ -23,12 +23,9 @@
 #include <nvrtc.h>
 
 #include <algorithm>
-#include <condition_variable>
 #include <cstdlib>
 #include <cstring>
-#include <deque>
 #include <map>
-#include <memory>
 #include <mutex>
 #include <set>
 #include <sstream>
@@ -672,74 +669,31 @@ static void hash_ops(Hash128& h, const DevOp* ops, int begin, int end) {
   }
 }
 
-// FP64 passes compile in the background: the first call with a structure runs
-// the interpreted kernels and queues the compile, the next call with it takes
-// the compiled kernel (waiting for it if it is not done yet), so a circuit that
-// runs once never waits.  Both kernels give the same bits.
+// FP64 passes compile on their second use: the first call with a structure runs
+// the interpreted kernels, the next one compiles (all its passes at once) and
+// later ones find the kernels, so a circuit that runs once never waits for a
+// compile.  Both kernels give the same bits.
 namespace {
-struct Job64 {
-  std::string src;
-  std::vector<char> cubin;
-  std::string log;
-  int state = 0;  // 0 queued or compiling, 1 done, 2 failed
-  uint64_t call = 0;
-};
-struct Background {
-  std::mutex mu;
-  std::condition_variable work, done;
-  std::deque<std::shared_ptr<Job64>> queue;
-  std::map<std::pair<uint64_t, uint64_t>, std::shared_ptr<Job64>> jobs;
-  std::vector<std::thread> threads;
-  bool stop = false;
-  void run() {
-    std::unique_lock<std::mutex> lk(mu);
-    while (true) {
-      work.wait(lk, [&] { return stop || !queue.empty(); });
-      if (stop) return;
-      auto j = queue.front();
-      queue.pop_front();
-      lk.unlock();
-      const bool ok = compile_one(j->src, j->cubin, j->log);
-      lk.lock();
-      j->state = ok ? 1 : 2;
-      j->src.clear();
-      done.notify_all();
-    }
-  }
-  void push(std::shared_ptr<Job64> j) {  // mu held
-    const size_t most = std::max(1u, std::thread::hardware_concurrency());
-    queue.push_back(j);
-    if (threads.size() < std::min(most, (size_t)64) && threads.size() < jobs.size()) threads.emplace_back([this] { run(); });
-    work.notify_one();
-  }
-  ~Background() {
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      stop = true;
-      work.notify_all();
-    }
-    for (auto& t : threads) t.join();  // (a compile in progress ends first)
-  }
-};
-Background& background() {
-  static Background b;
-  return b;
+constexpr size_t kSeenMax = size_t(1) << 16;  // structures remembered; then all are forgotten
+std::map<std::pair<uint64_t, uint64_t>, uint64_t>& seen64() {
+  static std::map<std::pair<uint64_t, uint64_t>, uint64_t> s;  // structure -> the call it was first seen in
+  return s;
 }
 }  // namespace
 
 int jit_pass_kernels64(int M, bool adj, const std::vector<JitPassRef64>& refs, std::vector<const void*>& out,
-                       uint64_t call, bool wait) {
+                       uint64_t call, bool at_once) {
   out.assign(refs.size(), nullptr);
   if (!jit_available()) return VQC_OK;
   const int flags[4] = {64, M, adj ? 1 : 0, jit_min_blocks64(adj)};
   std::vector<std::pair<uint64_t, uint64_t>> keys(refs.size());
-  std::vector<std::shared_ptr<Job64>> jobs(refs.size());
-  Background& bg = background();
+  std::vector<size_t> miss;
   {
-    std::lock_guard<std::mutex> lk(bg.mu);
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (seen64().size() > kSeenMax) seen64().clear();
     for (size_t i = 0; i < refs.size(); ++i) {
       const JitPassRef64& r = refs[i];
-      if (!r.stages) continue;
+      if (!r.stages || r.npool > kJitMaxCoef / 2) continue;
       Hash128 h;
       h.add(flags, sizeof(flags));
       h.val(r.nstages);
@@ -752,50 +706,28 @@ int jit_pass_kernels64(int M, bool adj, const std::vector<JitPassRef64>& refs, s
         hash_ops(h, r.ops, st.op_begin, st.op_end);
       }
       keys[i] = {h.a, h.b};
-      auto it = bg.jobs.find(keys[i]);
-      if (it != bg.jobs.end()) {
-        jobs[i] = it->second;
-        continue;
-      }
-      auto j = std::make_shared<Job64>();
-      j->src = jit_pass_source64(M, adj, r.stages, r.nstages, r.ops, r.npool);
-      j->call = call;
-      jobs[i] = bg.jobs[keys[i]] = j;
-      if (j->src.empty())
-        j->state = 2;
-      else
-        bg.push(j);
+      auto it = hcache().find(keys[i]);
+      if (it != hcache().end())
+        out[i] = it->second;
+      else if ((seen64().emplace(keys[i], call).first->second != call || at_once) &&
+               std::find_if(miss.begin(), miss.end(), [&](size_t m) { return keys[m] == keys[i]; }) == miss.end())
+        miss.push_back(i);
     }
   }
-  long long compiled = 0;
+  if (miss.empty()) return VQC_OK;
+  std::vector<std::string> srcs(miss.size());
+  for (size_t k = 0; k < miss.size(); ++k) {
+    const JitPassRef64& r = refs[miss[k]];
+    srcs[k] = jit_pass_source64(M, adj, r.stages, r.nstages, r.ops, r.npool);
+  }
+  std::vector<const void*> ks;
+  if (int rc = jit_kernels(srcs, ks, "vqc_pass64")) return rc;
+  std::lock_guard<std::mutex> lk(g_mu);
+  for (size_t k = 0; k < miss.size(); ++k) hcache()[keys[miss[k]]] = ks[k];  // (nullptr: failed; interpreted)
   for (size_t i = 0; i < refs.size(); ++i) {
-    if (!jobs[i] || (jobs[i]->call == call && !wait)) continue;
-    Job64& j = *jobs[i];
-    {
-      std::unique_lock<std::mutex> lk(bg.mu);
-      bg.done.wait(lk, [&] { return j.state != 0; });
-    }
-    std::lock_guard<std::mutex> lk(g_mu);
     auto it = hcache().find(keys[i]);
-    if (it != hcache().end()) {
-      out[i] = it->second;
-      continue;
-    }
-    cudaLibrary_t lib = nullptr;
-    cudaKernel_t k = nullptr;
-    const void* kernel = nullptr;
-    if (j.state == 1 &&
-        cudaLibraryLoadData(&lib, j.cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0) == cudaSuccess &&
-        cudaLibraryGetKernel(&k, lib, "vqc_pass64") == cudaSuccess)
-      kernel = (const void*)k;
-    else
-      cudaGetLastError();  // (the interpreted kernel runs the pass)
-    if (env_int("VQC_JIT_VERBOSE", 0)) fprintf(stderr, "vqc jit: %s\n", j.log.c_str());
-    std::vector<char>().swap(j.cubin);
-    out[i] = hcache()[keys[i]] = kernel;
-    ++compiled;
+    if (refs[i].stages && !out[i] && it != hcache().end()) out[i] = it->second;
   }
-  if (compiled) prof_note("jit_compiled_passes", compiled);
   return VQC_OK;
 }
 

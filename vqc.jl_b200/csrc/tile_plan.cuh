@@ -178,9 +178,8 @@ int jit_pass_kernels(int M, bool adj, const std::vector<JitPassRef>& refs, std::
                      bool batch = false, bool compile = true, int rb = kRegBits);
 
 // The same for FP64 passes (the classic plan).  `call` names the user's call
-// the passes belong to: a structure first seen in it runs interpreted while it
-// compiles in the background; one seen in an earlier call is waited for.
-// wait: compile at once.
+// the passes belong to: a structure first seen in it runs interpreted; one seen
+// in an earlier call is compiled.  at_once: compile at first sight.
 struct JitPassRef64 {
   const DevStage* stages = nullptr;
   int nstages = 0;
@@ -190,7 +189,7 @@ struct JitPassRef64 {
 int jit_min_blocks64(bool adj);
 std::string jit_pass_source64(int M, bool adj, const DevStage* stages, int nstages, const DevOp* ops, int npool);
 int jit_pass_kernels64(int M, bool adj, const std::vector<JitPassRef64>& refs, std::vector<const void*>& out,
-                       uint64_t call, bool wait);
+                       uint64_t call, bool at_once);
 
 // compiled: an FP32 packed plan with compiled batch kernels (fwd_k / adj_k)
 // when every pass has one already, else the classic plan for the generic
