@@ -10,13 +10,15 @@
 // gate of the pass to them, and writes them back: one HBM read + write per
 // pass instead of per gate.
 //   * a gate whose matrix acts on one or two target qubits (after stripping
-//     control qubits, read off the matrix) is applied in registers: each
-//     thread holds 16 amplitudes spanning 4 tile bits ("register bits"), and
-//     the pass is cut into *stages*, each with one register-bit set;
-//     between stages the tile goes through shared memory (XOR-swizzled, so
-//     the 16-byte / 8-byte accesses are free of bank conflicts);
-//   * controls on tile bits are tested per amplitude, controls on non-tile
-//     qubits once per tile;
+//     control qubits, read off the matrix) works on 4 tile bits ("register
+//     bits"): each thread owns the 16 amplitudes spanning them, in registers
+//     (compiled passes) or at its own places of the tile (interpreted ones),
+//     and the pass is cut into *stages*, each with one register-bit set;
+//     between stages the amplitudes change owners through shared memory
+//     (XOR-swizzled, so the 16-byte / 8-byte accesses are free of bank
+//     conflicts);
+//   * controls on thread bits are tested once per op, on register bits they
+//     select addresses, on non-tile qubits they are tested once per tile;
 //   * diagonal gates (CZ, CPHASE, ...) act on any qubits, tile or not;
 //   * consecutive one-qubit gates on the same qubit are merged into one 2x2.
 // In the reverse sweep (ADJ) each op applies U^dagger to both the cotangent
@@ -194,7 +196,9 @@ static TileConfig tile_config(int dtype, int n) {
   // tile qubits so that a tile is made of 128-byte runs (11-qubit FP32 tiles
   // for the reverse sweep measured slower: more passes at the same pass cost;
   // 3 always-resident FP32 qubits give 10 % fewer passes at 1.4x the reverse
-  // pass time, 11.6 vs 12.6 gradients/s at n = 26)
+  // pass time, 11.6 vs 12.6 gradients/s at n = 26; with 2^12 FP64
+  // amplitudes 256 threads wait for one another where 128 did: a 27-qubit
+  // circuit took 9.67 against 9.14 ms)
   const int M = std::min(dtype == VQC_C64 ? 12 : 11, n);
   return {M, std::min(dtype == VQC_C64 ? 4 : 3, M)};
 }
@@ -1714,9 +1718,12 @@ int serve_jit_gridx(int M, bool adj, const std::vector<const void*>& ks, const S
   return (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, grid));
 }
 
+size_t serve_pass_smem(int dtype, int M, bool adj, const PassShape& shape) {
+  return pass_smem(dtype == VQC_C64 ? sizeof(float2) : sizeof(double2), M, adj, shape);
+}
+
 int serve_launch_jit(int M, bool adj, const void* kernel, const TileItem* d_items, int nitems, int gridx,
-                     const PassShape& maxs, cudaStream_t stream) {
-  const size_t smem = pass_smem(sizeof(float2), M, adj, maxs);
+                     size_t smem, cudaStream_t stream) {
   int device = 0;
   VQC_CK(cudaGetDevice(&device));
   if (int rc = allow_smem(device, kernel)) return rc;
@@ -1732,14 +1739,13 @@ static const void* batch_kernel(int dtype, bool adj) {
 }
 
 int serve_tile_gridx(int dtype, int M, bool adj, const PassShape& maxs, int64_t max_ntiles, int device) {
-  const size_t smem = pass_smem(dtype == VQC_C64 ? 8 : 16, M, adj, maxs);
+  const size_t smem = serve_pass_smem(dtype, M, adj, maxs);
   const int g = kernel_grid(device, batch_kernel(dtype, adj), 1 << (M - kRegBits), smem);
   return (int)std::max<int64_t>(1, std::min<int64_t>(max_ntiles, g));
 }
 
 int serve_launch_tiles(int dtype, int M, bool adj, const TileItem* d_items, int nitems, int gridx,
-                       const PassShape& maxs, cudaStream_t stream) {
-  const size_t smem = pass_smem(dtype == VQC_C64 ? 8 : 16, M, adj, maxs);
+                       size_t smem, cudaStream_t stream) {
   const void* k = batch_kernel(dtype, adj);
   int device = 0;
   VQC_CK(cudaGetDevice(&device));

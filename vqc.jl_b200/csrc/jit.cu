@@ -1,4 +1,4 @@
-// Run-time specialised FP32 tile kernels.
+// Run-time specialised tile kernels: FP32 (packed), and FP64 (jit_pass_source64).
 //
 // The interpreted tile kernel (tile_f32.cuh, interp_ops) decodes every op of
 // a pass at run time; on sm_100 that costs about as many integer and move
@@ -15,8 +15,9 @@
 // reads them.
 //
 // VQC_JIT=0 / off: never (the generic tile kernel runs every pass); 1 / on:
-// every FP32 tile pass; auto (default): passes of states with at least 2^18
-// amplitudes; interp: the packed plan on its interpreter (testing).  If
+// every tile pass; auto (default): passes of FP32 states with at least 2^18
+// amplitudes and FP64 states with at least 2^20 (from a structure's second call
+// on); interp: the packed plan on its interpreter (testing).  If
 // NVRTC cannot be loaded the generic kernel runs; if one compilation fails,
 // that pass runs on the packed interpreter (both are GPU kernels).
 #include <dlfcn.h>
@@ -479,7 +480,8 @@ int jit_min_blocks64(bool adj) { return adj ? env_int("VQC_JIT_MINB_ADJ64", 2) :
 // device functions as the interpreted body (tile_ops.cuh), so both give the
 // same bits.  Measured against the interpreter on 2^23 amplitudes: reverse pass
 // 547 -> 337 us, forward 168 -> 106 us; U3 + CZ + Toffoli on 2^27: 5.0 -> 2.3 ms
-// per pass.  Bound by fetching the straight-line code and by the FP64 pipe.
+// per pass (1.5 ms with deferred phases and coalesced ends).  Bound by fetching
+// the straight-line code and by the FP64 pipe.
 std::string jit_pass_source64(int M, bool adj, const DevStage* st, int nst, const DevOp* ops, int npool) {
   if (npool > kJitMaxCoef / 2) return std::string();  // beyond the kernel-parameter space: interpreted
   std::ostringstream os;

@@ -476,21 +476,16 @@ static void worker_main(vqc_server_s* s) {
         const int M = std::get<0>(kv.first);
         const void* k = std::get<2>(kv.first);
         Group& g = kv.second;
-        PassShape mx;
-        mx.packed = k != nullptr;
+        size_t smem = 0;
         int gridx = 0;
         for (size_t i = 0; i < g.items.size(); ++i) {
-          const PassShape& sh = g.locs[i]->shape;
-          mx.nslots = std::max(mx.nslots, sh.nslots);
-          mx.nstages = std::max(mx.nstages, sh.nstages);
-          mx.nops = std::max(mx.nops, sh.nops);
-          mx.npool = std::max(mx.npool, sh.npool);
+          smem = std::max(smem, serve_pass_smem(s->dtype, M, adj != 0, g.locs[i]->shape));
           gridx = std::max(gridx, g.items[i].ncta);
         }
-        const int rc = k ? serve_launch_jit(M, adj != 0, k, (const TileItem*)g.d, (int)g.items.size(), gridx, mx,
+        const int rc = k ? serve_launch_jit(M, adj != 0, k, (const TileItem*)g.d, (int)g.items.size(), gridx, smem,
                                             s->stream)
                          : serve_launch_tiles(s->dtype, M, adj != 0, (const TileItem*)g.d, (int)g.items.size(),
-                                              gridx, mx, s->stream);
+                                              gridx, smem, s->stream);
         if (rc) {
           fail_all(s, vqc_last_error());
           return false;

@@ -203,11 +203,14 @@ void serve_compile_plan(const ReqPlan& packed, bool want_grad);
 // CTAs per request of the compiled batch kernels ks of a plan's passes.
 int serve_jit_gridx(int M, bool adj, const std::vector<const void*>& ks, const SerialPlan& sp, int64_t ntiles,
                     int device);
+// Shared memory of one request's pass; a batched launch takes the largest of
+// its items' (each CTA lays its own item out from the start).
+size_t serve_pass_smem(int dtype, int M, bool adj, const PassShape& shape);
 int serve_launch_jit(int M, bool adj, const void* kernel, const TileItem* d_items, int nitems, int gridx,
-                     const PassShape& maxs, cudaStream_t stream);
+                     size_t smem, cudaStream_t stream);
 int serve_tile_gridx(int dtype, int M, bool adj, const PassShape& maxs, int64_t max_ntiles, int device);
 int serve_launch_tiles(int dtype, int M, bool adj, const TileItem* d_items, int nitems, int gridx,
-                       const PassShape& maxs, cudaStream_t stream);
+                       size_t smem, cudaStream_t stream);
 int serve_launch_reduce(const RedItem* d_items, int nitems, int maxslots, cudaStream_t stream);
 void contract_grads(const std::vector<AccRef>& accs, const double* A, double* grads);
 
