@@ -21,7 +21,7 @@ def test_same_bits(monkeypatch):
     """Every kind of gate, forward and in the reverse sweep: the first call
     (interpreted) and the later ones (compiled)."""
     monkeypatch.delenv("VQC_JIT", raising=False)
-    n = 20  # the smallest size that compiles by default
+    n = 23  # the smallest size that compiles by default
     rng = np.random.default_rng(500)
     c, _ = random_mixed_circuit(rng, n, 40, with_wide=False)
     psi0, target = rand_psi(rng, n), rand_psi(rng, n)
@@ -39,7 +39,7 @@ def test_same_bits(monkeypatch):
 def test_calls_agree_across_the_compile(monkeypatch):
     """The default mode at a size that compiles: interpreted, then compiled."""
     monkeypatch.delenv("VQC_JIT", raising=False)
-    n, layers = 20, 2
+    n, layers = 23, 2
     rng = np.random.default_rng(510)
     c = W.to_circuit(W.rxyz_crx_spec(n, layers, rng.uniform(0, 2 * np.pi, layers * (4 * n - 1))))
     H, s = W.to_operator(W.xxz_spec(n, 0.5)), V.StateVector(n)

@@ -51,9 +51,8 @@ def test_crowded_passes(dtype, n, kind):
     c, H = crowded(rng, min(n, 11), kind), W.to_operator(W.xxz_spec(n, 0.5))
     psi = rand_psi(rng, n)
     s = V.StateVector(psi.astype(dtype), dtype=dtype)
-    for _ in range(2):  # (FP64 from 20 qubits: interpreted, then compiled)
-        got = V.apply(c, V.StateVector(psi.astype(dtype), dtype=dtype))
-        e, g = V.energy_and_gradient(H, c, s)
+    got = V.apply(c, V.StateVector(psi.astype(dtype), dtype=dtype))
+    e, g = V.energy_and_gradient(H, c, s)
     assert max_abs(got.storage(), O.apply_circuit(as_input(psi, dtype), reference(c), nthreads=4)) < tol(dtype)
     e_ref, g_ref = O.energy_and_gradient(reference(c), O.terms_from_spec(W.xxz_spec(n, 0.5)), as_input(psi, dtype),
                                          nthreads=4)

@@ -196,9 +196,9 @@ static TileConfig tile_config(int dtype, int n) {
   // tile qubits so that a tile is made of 128-byte runs (11-qubit FP32 tiles
   // for the reverse sweep measured slower: more passes at the same pass cost;
   // 3 always-resident FP32 qubits give 10 % fewer passes at 1.4x the reverse
-  // pass time, 11.6 vs 12.6 gradients/s at n = 26; with 2^12 FP64
-  // amplitudes 256 threads wait for one another where 128 did: a 27-qubit
-  // circuit took 9.67 against 9.14 ms)
+  // pass time, 11.6 vs 12.6 gradients/s at n = 26; 2^12 FP64
+  // amplitudes, a tenth fewer passes: 9.67 against 9.72 ms for a 27-qubit
+  // circuit, 3.66 against 3.65 ms for a 23-qubit gradient, and 128 KB of tiles)
   const int M = std::min(dtype == VQC_C64 ? 12 : 11, n);
   return {M, std::min(dtype == VQC_C64 ? 4 : 3, M)};
 }
@@ -1180,10 +1180,19 @@ static bool use_jit(const vqc_state h) {
 // The packed FP32 plan layout: for the compiled passes, or forced with
 // VQC_JIT=interp (the packed interpreter, the compiled kernels' fallback).
 static bool use_packed(const vqc_state h) { return h->dtype == VQC_C64 && (use_jit(h) || jit_mode() == 3); }
-// Compiled FP64 passes: states of at least 2^20 amplitudes (auto), all (on).
-static bool use_jit64(const vqc_state h) {
+// FP64 states planned for compiled passes (deferred phases): at least 2^20
+// amplitudes (auto), all (on); compiled: at least 2^kCompileQubits64.
+// Smaller states run such plans interpreted: compiling a call's passes takes the
+// host some seconds and saves 2 ms a call at 23 qubits but 0.2 ms at 20, and a
+// stream of different circuits of 20-22 qubits met a compile in most calls (5
+// against 400 requests a second).
+constexpr int kCompileQubits64 = 23;
+static bool plans_like_jit64(const vqc_state h) {
   const int mode = jit_mode();
   return h->dtype == VQC_C128 && (mode == 1 || (mode == 2 && h->nq >= 20)) && jit_available();
+}
+static bool use_jit64(const vqc_state h) {
+  return plans_like_jit64(h) && (jit_mode() == 1 || h->nq >= kCompileQubits64);
 }
 static uint64_t new_call() {
   static std::atomic<uint64_t> n{0};
@@ -1274,7 +1283,7 @@ static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& pa
                          : kernel_grid(h->device, tile_kernel<R, ADJ>(M, locs[pi].shape), 1 << (M - kRegBits), smem);
     // the CTAs' partial sums group alike in both kernels of an FP64 pass
     if constexpr (ADJ && std::is_same<R, double>::value)
-      if (use_jit64(h)) g = device_info(h->device).sms * jit_min_blocks64(true);
+      if (plans_like_jit64(h)) g = device_info(h->device).sms * jit_min_blocks64(true);
     grids[pi] = (int)std::min<int64_t>(g, locs[pi].ntiles);
   }
   // partial sums scratch: one row of 8 doubles per (CTA, slot) of every pass,
@@ -1387,7 +1396,7 @@ static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const do
       return analyze_gate(h->nq, gates[bad[t]].nq, gates[bad[t]].pos, mats + gates[bad[t]].mat, false, specs[bad[t]]);
   std::vector<PlanPass> passes;
   plan_passes(h->nq, tile_config(h->dtype, h->nq), false, items, passes);
-  if (defer && (use_packed(h) || use_jit64(h))) defer_phases(h->nq, false, h->dtype == VQC_C64, passes);
+  if (defer && (use_packed(h) || plans_like_jit64(h))) defer_phases(h->nq, false, h->dtype == VQC_C64, passes);
   const uint64_t call = new_call();
   const char* pc = std::getenv("VQC_PLAN_CHUNKS");  // 0: one serialisation for the whole sweep
   if (passes.size() < 4 || (pc && *pc && std::atoi(pc) == 0))
@@ -1480,7 +1489,7 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
   std::vector<PItem> items = reverse_items(specs, params);
   std::vector<PlanPass> passes;
   plan_passes(h->nq, tile_config(h->dtype, h->nq), true, items, passes);
-  if (use_packed(h) || use_jit64(h)) defer_phases(h->nq, true, h->dtype == VQC_C64, passes);
+  if (use_packed(h) || plans_like_jit64(h)) defer_phases(h->nq, true, h->dtype == VQC_C64, passes);
   // standalone gates with parameters: split their passes out so the per-gate
   // path can evaluate the partials right after the uncompute
   std::vector<AccRef> accs;

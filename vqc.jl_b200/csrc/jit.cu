@@ -16,7 +16,7 @@
 //
 // VQC_JIT=0 / off: never (the generic tile kernel runs every pass); 1 / on:
 // every tile pass; auto (default): passes of FP32 states with at least 2^18
-// amplitudes and FP64 states with at least 2^20 (from a structure's second call
+// amplitudes and FP64 states with at least 2^23 (from a structure's second call
 // on); interp: the packed plan on its interpreter (testing).  If
 // NVRTC cannot be loaded the generic kernel runs; if one compilation fails,
 // that pass runs on the packed interpreter (both are GPU kernels).
@@ -674,7 +674,9 @@ static void hash_ops(Hash128& h, const DevOp* ops, int begin, int end) {
 // FP64 passes compile on their second use: the first call with a structure runs
 // the interpreted kernels, the next one compiles (all its passes at once) and
 // later ones find the kernels, so a circuit that runs once never waits for a
-// compile.  Both kernels give the same bits.
+// compile; neither does one that shares some passes with an earlier one (a
+// chunk of the sweep with a pass not seen before compiles nothing).  Both
+// kernels give the same bits.
 namespace {
 constexpr size_t kSeenMax = size_t(1) << 16;  // structures remembered; then all are forgotten
 std::map<std::pair<uint64_t, uint64_t>, uint64_t>& seen64() {
@@ -688,6 +690,7 @@ int jit_pass_kernels64(int M, bool adj, const std::vector<JitPassRef64>& refs, s
   out.assign(refs.size(), nullptr);
   if (!jit_available()) return VQC_OK;
   const int flags[4] = {64, M, adj ? 1 : 0, jit_min_blocks64(adj)};
+  bool all_seen = true;
   std::vector<std::pair<uint64_t, uint64_t>> keys(refs.size());
   std::vector<size_t> miss;
   {
@@ -711,12 +714,13 @@ int jit_pass_kernels64(int M, bool adj, const std::vector<JitPassRef64>& refs, s
       auto it = hcache().find(keys[i]);
       if (it != hcache().end())
         out[i] = it->second;
-      else if ((seen64().emplace(keys[i], call).first->second != call || at_once) &&
-               std::find_if(miss.begin(), miss.end(), [&](size_t m) { return keys[m] == keys[i]; }) == miss.end())
+      else if (seen64().emplace(keys[i], call).first->second == call && !at_once)
+        all_seen = false;
+      else if (std::find_if(miss.begin(), miss.end(), [&](size_t m) { return keys[m] == keys[i]; }) == miss.end())
         miss.push_back(i);
     }
   }
-  if (miss.empty()) return VQC_OK;
+  if (miss.empty() || !all_seen) return VQC_OK;
   std::vector<std::string> srcs(miss.size());
   for (size_t k = 0; k < miss.size(); ++k) {
     const JitPassRef64& r = refs[miss[k]];
