@@ -208,14 +208,17 @@ __device__ __forceinline__ void tile_body(const TileItem& it) {
       int o = S->op_begin, held = -1;  // held: the slot of an op whose sums wait for a second op's
       R ha[4];
       const int4* words = reinterpret_cast<const int4*>(x.ops + o);
-      int4 w0 = words[0], w1 = words[1];  // (read one op ahead; the word after the last op is in the tables)
+      // read one op ahead, never past the pass's ops: a coalesced end stage has none,
+      // and behind them the launch may have asked for one matrix's word only
+      int4 w0 = make_int4(0, 0, 0, 0), w1 = w0;
+      if (o < oe && VQC_DCHECK(o, it.p.nops)) w0 = words[0], w1 = words[1];
 #pragma unroll 1
       for (; o < oe; ++o) {
         const DevOp* op = x.ops + o;
         const int4 cur = w0;
         const OpWord ow(w1);
         words += sizeof(DevOp) / 16;
-        if (o + 1 < oe) w0 = words[0], w1 = words[1];
+        if (o + 1 < oe && VQC_DCHECK(o + 1, it.p.nops)) w0 = words[0], w1 = words[1];
         const int code = cur.x, sel = (code >> kSelShift) & 127;
         if (code & kCodeGCtl) {  // a control on a non-tile qubit: uniform over the tile
           if ((x.base & op->gmask) != op->gval) continue;
