@@ -129,7 +129,7 @@ int apply_gate_raw(vqc_state h, int k, const int* pos, const double* mat);
 int dm_apply_gate_raw(vqc_state h, int k, const int* pos, const double* mat);
 
 // The fused tile engine (fused.cu).  Plans the gates into passes and runs them.
-// defer: phases may be deferred from gate to gate (see defer_phases).
+// defer: phases may be deferred from gate to gate (see Deferred, fused.cu).
 int apply_circuit_fused(vqc_state h, const vqc_gate* gates, int ngates, const double* mats, bool defer = true);
 
 inline int64_t mask_of(int k, const int* sp, int nq, int64_t* mask) {

@@ -33,6 +33,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <optional>
 #include <mutex>
 #include <set>
 #include <thread>
@@ -177,7 +178,6 @@ struct PlanPass {
   std::vector<FOp> ops;
   std::vector<PlanStage> stages;
   int nslots = 0;
-  double norm0 = 1;              // the deferred norm when the pass starts (defer_phases)
 };
 
 static void tile_bits(const PlanPass& p, int (&tbit)[64]) {
@@ -288,145 +288,169 @@ static void plan_passes(int n, const TileConfig& tc, bool adj, std::vector<PItem
   }
 }
 
-// Phases deferred.  A 2x2 M with |m00| = |m11| is a diag(1, p) T, a = m00, |p| = 1,
-// T = [[1, x], [y, 1]], and T takes half the products of a general 2x2 (8
-// instead of 16 FMAs per pair of amplitudes); the tile passes are bound by their
-// arithmetic.  The phase p stays behind as a pending diag(1, p) on the qubit and
-// a as a factor g of the whole state.  A pending phase passes a control and a
-// diagonal gate unchanged, turns another gate on its qubit into one with rotated
-// off-diagonal entries, and is absorbed by the next uncontrolled one-qubit gate
-// there; the last such gate (before the end of the circuit, or a gate outside
-// the tile passes) takes its whole matrix and g, so no pass is added.  The first
-// deferred gate of a pass takes the norm of g (real diagonal, 12 FMAs), so that
-// amplitudes grow over one pass only.  With U3 + CZ every dense gate but the last
-// layer's costs half; with CRX ladders the controlled gates cost 6 instead of 4
-// per pair, the merged rotations 8 instead of 16.
+// Phases deferred.  A 2x2 M = c U, U unitary with |m00| = |m11|, is a diag(1, p) T,
+// a = m00, |p| = 1, T = [[1, x], [-conj(x), 1]], and T takes half the products of a
+// general 2x2 (8 instead of 16 FMAs per pair of amplitudes); the tile passes are
+// bound by their arithmetic.  The phase p stays behind as a pending diag(1, p) on
+// the qubit and a as a factor g of the whole state.  A pending phase passes a
+// control and a diagonal gate unchanged, turns another gate on its qubit into one
+// with rotated off-diagonal entries, and is absorbed by the next uncontrolled
+// one-qubit gate there; the last such gate (before the end of the circuit, or a
+// gate outside the tile passes) takes its whole matrix and g, so no pass is added.
+//
+// The amplitudes in flight are the true ones times 1 / |g|, so |g| is bounded: the
+// first deferred gate of a pass and every kNormEvery-th after it take the norm of g
+// (real diagonal, 12 FMAs), and so does one that would take |g| out of the window
+// [kNormMin, 1 / kNormMin].  The gates are walked in the order they run, stage by
+// stage: a stage runs every layer of its few register qubits, so in any other order
+// (the planner's, 192 ops to a pass) the factors of one qubit pair's forty layers
+// would meet before the gates meant to take them.  A deferred gate's factor is
+// |cos| of a half angle, one half in the geometric mean: 2^-8 between two norms in
+// FP32, whose reverse sweep sums products of two such amplitudes; the window is
+// reached by chance less than once in 10^5 runs of eight random gates, by gates
+// near X (RX(pi)) at once.
 //
 // Which form a gate takes depends on its place alone, not on its angle (but for
-// |m00| < kMinPivot and exact zeros), so that new angles reuse compiled passes.
-// T is a multiple of a unitary whatever |x|: a large x is as accurate as a small one.
+// the window, |m00| < kMinPivot and exact zeros), so that new angles reuse compiled
+// passes.  T is a multiple of a unitary whatever |x|: a large x is as accurate as a
+// small one.
 //
 // Only where the passes are compiled (states of 2^18 FP32, 2^20 FP64 amplitudes
 // and more): the interpreted ones are bound by latency, and a CNOT that was a
 // swap of two loads becomes a product (serving's reverse launches 66 -> 81 us).
 // Measured: reverse pass 1,060 -> 957 us and forward 350 -> 325 us at 2^26 FP32,
 // U3 + CZ + Toffoli pass 7.9 -> 5.6 ms at 2^30 FP32 and 2.3 -> 1.75 ms at 2^27 FP64.
-// Accuracy against FP64 (16 circuits of 20 layers on 20 qubits, FP32): gradient
-// 5.6e-7 (1.04e-6 with whole matrices), norm 1.4e-7 (3.1e-7), energy as before
-// (1.7e-7, 2.0e-7 absolute): the rounding of the angles, not of the amplitudes,
-// decides it.  The FP32 gradient's own forward sweep keeps whole matrices (its
-// passes gain 2 % of the gradient's time), so that sweep's energy is unchanged.
-// In FP32 x is rounded first and y = -conj(x), so that this holds exactly.
+// Accuracy: T is taken from the unitary nearest to M; g, p and the products with them
+// are kept in long double and every entry is rounded once; x is rounded before
+// -conj(x) is formed and g takes up the change of modulus, so T is a multiple of a
+// unitary exactly.  Against 80-bit arithmetic (13 qubits, 12 circuits each of RX RY RZ +
+// CRX, RY RZ + CNOT, U3 + CZ + Toffoli and U3 + CNOT; whole matrices in brackets):
+// FP32 state 4.0 to 4.5e-7 (4.1 to 4.6e-7), gradient 3.8 to 5.8e-7 (4.8 to 6.6e-7);
+// FP64 state 1.1 to 2.2e-15 (1.0 to 2.2e-15), gradient 2.2e-15 (2.0 to 2.7e-15).  The FP32 gradient's
+// own forward sweep keeps whole matrices (its passes gain 2 % of the gradient's
+// time), so that sweep's energy is unchanged.
 //
 // The reverse sweep applies the same ops to both states, so its reduced
 // matrices come out in the pending frame: A[a][b] = |g|^2 conj(p_a) p_b A'[a][b]
-// over the op's target.  The phases are folded into the D matrices here; |g| is
-// the product over the ops that have run, in the order of the pass's stages
-// (AccRef::scale).
-constexpr double kMinPivot = 1e-9, kMinScale = 1e-15;  // (amplitudes grow by 1 / |g|)
-// A phase within rounding of 1, i, -1 or -i is that one (a rounding error must
-// not decide which form the next gates take).
-static cd whole_turns(cd p) {
-  for (const cd& q : {cd(1), cd(-1), cd(0, 1), cd(0, -1)})
-    if (std::abs(p - q) < 1e-14) return q;
-  return p;
-}
-static void defer_phases(int n, bool adj, bool f32, std::vector<PlanPass>& passes) {
-  for (const PlanPass& p : passes)
-    if (adj && p.standalone) return;  // (their reduced matrices are taken in the plain frame)
-  // the ops on each qubit that a later uncontrolled one-qubit op follows
-  std::vector<char> later;  // by op, in order
-  {
+// over the op's target.  The phases are folded into the D matrices here; |g| when
+// the op has run is FOp::norm (AccRef::scale is its square).
+constexpr double kMinPivot = 1e-9;
+using cl = std::complex<long double>;
+class Deferred {
+ public:
+  // Marks the ops of the sweep that a later uncontrolled one-qubit op on their qubit follows.
+  Deferred(int n, bool adj, bool f32, std::vector<PlanPass>& passes)
+      : adj_(adj), f32_(f32), every_(f32 ? 8 : 32), min_(f32 ? 1e-12 : 1e-60), tol_(f32 ? 1e-13 : 1e-14),
+        least_(f32 ? 1e-30 : 1e-280), ph_(n, cl(1)) {
     std::vector<char> open(n, 0);
-    size_t total = 0;
-    for (const PlanPass& p : passes) total += p.ops.size();
-    later.assign(total, 0);
-    size_t k = total;
     for (size_t pi = passes.size(); pi-- > 0;) {
-      const PlanPass& p = passes[pi];
+      PlanPass& p = passes[pi];
       if (p.standalone) {
         std::fill(open.begin(), open.end(), 0);
         continue;
       }
       for (size_t i = p.ops.size(); i-- > 0;) {
-        const FOp& f = p.ops[i];
-        --k;
+        FOp& f = p.ops[i];
         if (f.kind != kOpU1 || f.cmask) continue;
-        later[k] = open[f.tq[0]];
+        f.later = open[f.tq[0]];
         open[f.tq[0]] = 1;
       }
     }
   }
-  std::vector<cd> ph(n, cd(1));
-  cd g(1);
-  size_t k = 0;
-  auto in_frame = [&](FOp& f) {  // the reduced matrix's frame, after the op
-    if (!adj || !f.acc || f.kind != kOpU1) return;
-    const cd p = ph[f.tq[0]];
-    if (p != cd(1))
-      for (PGrad& pg : f.grads) pg.D[1] *= p, pg.D[2] *= std::conj(p);
-  };
-  for (PlanPass& pass : passes) {
-    bool first = true;  // no deferred gate in this pass yet
-    pass.norm0 = std::abs(g);
-    for (FOp& f : pass.ops) {
-      const double before = std::abs(g);
-      const bool absorbed = later[k++];
-      if (f.kind == kOpU2) {
-        const cd a = ph[f.tq[0]], b = ph[f.tq[1]];
-        if (a != cd(1) || b != cd(1)) {
-          const cd c[4] = {cd(1), a, b, a * b};
-          for (int r = 0; r < 4; ++r)
-            for (int q = 0; q < 4; ++q)
-              if (f.mat[4 * r + q] != cd(0)) f.mat[4 * r + q] *= c[q] * std::conj(c[r]);
-        }
-      } else if (f.kind == kOpU1) {
-        cd& p = ph[f.tq[0]];
-        Mat& m = f.mat;
-        if (f.cmask) {
-          if (p != cd(1)) {
-            if (m[1] != cd(0)) m[1] *= p;
-            if (m[2] != cd(0)) m[2] *= std::conj(p);
-          }
-        } else {
-          if (p != cd(1)) m[1] *= p, m[3] *= p;
-          const cd a = m[0];
-          const double na = std::abs(a), nb = std::abs(m[3]);
-          const double top = std::max(std::max(na, nb), std::max(std::abs(m[1]), std::abs(m[2])));
-          if (absorbed && std::min(na, nb) > kMinPivot * top && std::abs(na - nb) <= 1e-13 * top) {
-            const cd np = whole_turns((m[3] / nb) * std::conj(a / na));
-            cd x = m[1] / a, y = m[2] / (a * np);
-            double s = 1;
-            if (f32 && std::abs(y + std::conj(x)) <= 1e-13 * (1 + std::abs(x))) {
-              const cd xr((float)x.real(), (float)x.imag());
-              s = std::sqrt((1 + std::norm(x)) / (1 + std::norm(xr)));
-              x = xr;
-              y = -std::conj(xr);
-            }
-            p = np;
-            g *= a * s;
-            const double ng = std::abs(g);
-            if (first || ng < kMinScale) {
-              m = {cd(ng), ng * x, ng * y, cd(ng)};
-              g /= ng;
-              f.form = kFormRC;
-            } else {
-              m = {cd(1), x, y, cd(1)};
-              f.form = x == cd(0) && y == cd(0) ? kFormId : kFormUD;
-            }
-            first = false;
-          } else {
-            for (cd& v : m) v *= g;
-            g = cd(1);
-            p = cd(1);
-          }
-        }
+  // A reverse sweep with gates outside the tile passes defers nothing: their
+  // reduced matrices are taken in the plain frame.
+  static bool applies(bool adj, const std::vector<PlanPass>& passes) {
+    for (const PlanPass& p : passes)
+      if (adj && p.standalone) return false;
+    return true;
+  }
+  // The sweep's next pass, its stages formed.
+  void pass(PlanPass& p) {
+    since_ = every_;  // (the pass's first deferred gate takes the norm)
+    for (const PlanStage& st : p.stages)
+      for (int oi : st.ops) op(p.ops[oi]);
+  }
+
+ private:
+  void op(FOp& f) {
+    Mat& m = f.mat;
+    if (f.kind == kOpU2) {
+      const cl a = ph_[f.tq[0]], b = ph_[f.tq[1]];
+      if (a != cl(1) || b != cl(1)) {
+        const cl c[4] = {cl(1), a, b, a * b};
+        for (int r = 0; r < 4; ++r)
+          for (int q = 0; q < 4; ++q)
+            if (m[4 * r + q] != cd(0)) m[4 * r + q] = cd(cl(m[4 * r + q]) * c[q] * std::conj(c[r]));
       }
-      in_frame(f);
-      f.gain = std::abs(g) / before;
+    } else if (f.kind == kOpU1 && f.cmask) {
+      const cl p = ph_[f.tq[0]];
+      if (p != cl(1)) {
+        if (m[1] != cd(0)) m[1] = cd(cl(m[1]) * p);
+        if (m[2] != cd(0)) m[2] = cd(cl(m[2]) * std::conj(p));
+      }
+    } else if (f.kind == kOpU1) {
+      one_qubit(f);
+    }
+    f.norm = (double)std::abs(g_);
+    if (adj_ && f.acc && f.kind == kOpU1) {  // the reduced matrix's frame
+      const cl p = ph_[f.tq[0]];
+      if (p != cl(1))
+        for (PGrad& pg : f.grads) pg.D[1] = cd(cl(pg.D[1]) * p), pg.D[2] = cd(cl(pg.D[2]) * std::conj(p));
     }
   }
-}
+  void one_qubit(FOp& f) {
+    cl& p = ph_[f.tq[0]];
+    const cl m0(f.mat[0]), m1 = cl(f.mat[1]) * p, m2(f.mat[2]), m3 = cl(f.mat[3]) * p;
+    const long double n0 = std::abs(m0), n1 = std::abs(m1), n2 = std::abs(m2), n3 = std::abs(m3);
+    const long double top = std::max(std::max(n0, n3), std::max(n1, n2));
+    const long double c = (n0 + n3) / 2, s = (n1 + n2) / 2, ng = std::abs(g_) * c;
+    if (f.later && std::min(n0, n3) > kMinPivot * top && std::abs(n0 - n3) <= tol_ * top &&
+        std::abs(n1 - n2) <= tol_ * top && ng > least_ && ng < 1 / least_) {
+      // The unitary nearest to M / |.|: the entries' phases, of moduli c, s, s, c,
+      // satisfy arg m1 + arg m2 = arg m0 + arg m3 + pi but for the rounding r of the
+      // matrix, which is shared out (taking any three entries as they are would put
+      // all of it into the fourth)
+      cl e0 = m0 / n0, e3 = m3 / n3, x(0);
+      long double r = 0;
+      if (n1 > 0 && n2 > 0) {
+        cl e1 = m1 / n1;
+        r = std::arg(-e1 * (m2 / n2) * std::conj(e0 * e3));
+        const long double cc = c * c / (c * c + s * s);
+        const cl d = std::polar(1.0L, r * (1 - cc) / 2);
+        e0 *= d, e3 *= d, e1 *= std::polar(1.0L, -r * cc / 2);
+        x = e1 * std::conj(e0) * (s / c);
+      }
+      if (std::abs(r) * s <= tol_ * top) {
+        p = whole_turns(e3 * std::conj(e0));
+        g_ *= e0 * c;
+        const bool whole = since_ >= every_ || ng < min_ || ng > 1 / min_;
+        const long double d = whole ? rounded(ng) : 1.0L;
+        const cl w(rounded(d * x.real()), rounded(d * x.imag()));
+        g_ *= std::sqrt((1 + std::norm(x)) / (1 + std::norm(w / d))) / d;
+        since_ = whole ? 0 : since_ + 1;
+        f.form = whole ? kFormRC : (w == cl(0) ? kFormId : kFormUD);
+        f.mat = {cd(d), cd(w), -std::conj(cd(w)), cd(d)};
+        return;
+      }
+    }
+    f.mat = {cd(m0 * g_), cd(m1 * g_), cd(m2 * g_), cd(m3 * g_)};
+    g_ = cl(1);
+    p = cl(1);
+  }
+  long double rounded(long double v) const { return f32_ ? (long double)(float)v : (long double)(double)v; }
+  // A phase within rounding of 1, i, -1 or -i is that one (a rounding error must
+  // not decide which form the next gates take).
+  cl whole_turns(cl p) const {
+    for (const cl& q : {cl(1), cl(-1), cl(0, 1), cl(0, -1)})
+      if (std::abs(p - q) < tol_ / 10) return q;
+    return p;
+  }
+  bool adj_, f32_;
+  int every_, since_ = 0;
+  long double min_, tol_, least_;  // (least_: a norm a matrix entry can hold)
+  std::vector<cl> ph_;
+  cl g_ = cl(1);
+};
 
 // Conflict check of a register-bit set for the shared-memory swizzle.
 // FP64: 16-byte amplitudes, quarter-warps over the tile swizzle Swz<double>;
@@ -832,8 +856,8 @@ struct StageTables {
 // One stage of the FP32 (packed) tile body: its DevStageF tables, its ops
 // (j-bit targets, register controls as compile-time cases or a mask, the
 // coefficient layouts of tile_f32.cuh) and their pool blocks.
-static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t tile_mask, const int (&tbit)[64], bool adj, int& slot, double& norm, int row, std::vector<DevStageF>& ds,
-                      std::vector<DevOp>& dops, std::vector<float2>& pool, size_t pool_begin,
+static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t tile_mask, const int (&tbit)[64], bool adj,
+                      int& slot, int row, std::vector<DevStageF>& ds, std::vector<DevOp>& dops, std::vector<float2>& pool, size_t pool_begin,
                       std::vector<AccRef>* accs, int rb) {
   DevStageF s{};
   const std::vector<int>& rs = st.rs;  // ascending, rs[0] = tile bit 0
@@ -868,7 +892,6 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t ti
   s.op_begin = (int)dops.size();
   for (int oi : st.ops) {
     const FOp& f = p.ops[oi];
-    norm *= f.gain;
     DevOp o{};
     o.code = f.kind;
     o.slot = -1;
@@ -957,10 +980,10 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t ti
         DevOp a = o;
         a.code = (a.code & ~15) | kOpAccD;
         dops.push_back(a);
-        if (accs) accs->push_back(AccRef{row + o.slot, f.grads, norm * norm});
+        if (accs) accs->push_back(AccRef{row + o.slot, f.grads, f.norm * f.norm});
         continue;
       }
-      if (accs) accs->push_back(AccRef{row + o.slot, f.grads, norm * norm, (o.code & kCodeAH) != 0});
+      if (accs) accs->push_back(AccRef{row + o.slot, f.grads, f.norm * f.norm, (o.code & kCodeAH) != 0});
       o.code |= kCodeAcc;
     }
     dops.push_back(o);
@@ -971,7 +994,7 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t ti
 
 template <class R, int M, bool ADJ>
 static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, SerialPlan& sp, std::vector<AccRef>* accs,
-                           bool packed = false, int rb = kRegBits) {
+                           Deferred* defer, bool packed = false, int rb = kRegBits) {
   Device d;
   std::vector<cplx<R>> pool;
   std::vector<PassLoc>& locs = sp.locs;
@@ -985,6 +1008,8 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
       continue;
     }
     plan_stages(p, M, dtype, packed, rb);
+    if (defer) defer->pass(p);
+    for (const FOp& f : p.ops) sp.norm_lo = std::min(sp.norm_lo, f.norm), sp.norm_hi = std::max(sp.norm_hi, f.norm);
     if (n >= kCoalesceQubits) coalesce_ends(p, M, dtype, packed, rb);
     std::vector<DevStage> ds;
     std::vector<DevOp> dops;
@@ -993,14 +1018,13 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
     uint64_t tile_mask = 0;
     for (int q : p.tile_q) tile_mask |= 1ull << q;
     int slot = 0;
-    double norm = p.norm0;
     while ((pool.size() * sizeof(cplx<R>)) % 16) pool.push_back(mkc<R>(R(0), R(0)));
     const size_t pool_begin = pool.size();
     std::vector<DevStageF> dsf;
     for (const PlanStage& st : p.stages) {
       if constexpr (std::is_same<R, float>::value) {
         if (packed) {
-          stage_f32(p, st, M, tile_mask, tbit, ADJ, slot, norm, row, dsf, dops, pool, pool_begin, accs, rb);
+          stage_f32(p, st, M, tile_mask, tbit, ADJ, slot, row, dsf, dops, pool, pool_begin, accs, rb);
           continue;
         }
       }
@@ -1025,7 +1049,6 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
       s.op_begin = (int)dops.size();
       for (int oi : st.ops) {
         const FOp& f = p.ops[oi];
-        norm *= f.gain;
         DevOp o{};
         o.code = f.kind;
         o.slot = -1;
@@ -1093,10 +1116,10 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
             a.cmask = a.cval = 0;
             a.gmask = a.gval = 0;
             dops.push_back(a);
-            if (accs) accs->push_back(AccRef{row + o.slot, f.grads, norm * norm});
+            if (accs) accs->push_back(AccRef{row + o.slot, f.grads, f.norm * f.norm});
             continue;
           }
-          if (accs) accs->push_back(AccRef{row + o.slot, f.grads, norm * norm, (o.code & kCodeAH) != 0});
+          if (accs) accs->push_back(AccRef{row + o.slot, f.grads, f.norm * f.norm, (o.code & kCodeAH) != 0});
           o.code |= kCodeAcc;
         }
         dops.push_back(o);
@@ -1140,7 +1163,7 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
 }
 
 static void note_plan(bool adj, const std::vector<PlanPass>& passes) {
-  long long np = 0, ns = 0, no = 0, nsa = 0;
+  long long np = 0, ns = 0, no = 0, nsa = 0, nd = 0;
   for (auto& p : passes) {
     if (p.standalone) {
       ++nsa;
@@ -1149,11 +1172,13 @@ static void note_plan(bool adj, const std::vector<PlanPass>& passes) {
     ++np;
     ns += (long long)p.stages.size();
     no += (long long)p.ops.size();
+    for (const FOp& f : p.ops) nd += f.form >= 0;
   }
   prof_note(adj ? "plan_adjoint_passes" : "plan_forward_passes", np);
   prof_note(adj ? "plan_adjoint_stages" : "plan_forward_stages", ns);
   prof_note(adj ? "plan_adjoint_ops" : "plan_forward_ops", no);
   prof_note("plan_standalone_gates", nsa);
+  prof_note(adj ? "plan_adjoint_deferred" : "plan_forward_deferred", nd);
 }
 
 template <int M, bool ADJ>
@@ -1223,7 +1248,7 @@ static size_t op_bytes_bound(const PlanPass& p) {
 // chunks of one sweep can be uploaded while these passes run.
 template <class R, int M, bool ADJ>
 static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& passes, const std::vector<GateSpec>& specs,
-                    std::vector<AccRef>* accs, double* rows_dev, uint64_t call, size_t op_off = 0,
+                    std::vector<AccRef>* accs, double* rows_dev, uint64_t call, Deferred* defer, size_t op_off = 0,
                     size_t* op_used = nullptr) {
   const int n = h->nq;
   SerialPlan sp;
@@ -1232,7 +1257,13 @@ static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& pa
   // four free register bits per stage; the generic kernels take 16
   int rb = (!ADJ && packed && use_jit(h) && wide_forward()) ? kWideRegBits : kRegBits;
   const size_t accs0 = accs ? accs->size() : 0;
-  serialize_plan<R, M, ADJ>(n, h->dtype, passes, sp, accs, packed, rb);
+  std::vector<PlanPass> plain;  // (to plan again at 16 amplitudes)
+  std::optional<Deferred> before;
+  if (rb != kRegBits) {
+    plain = passes;
+    if (defer) before = *defer;
+  }
+  serialize_plan<R, M, ADJ>(n, h->dtype, passes, sp, accs, defer, packed, rb);
   note_plan(ADJ, passes);
   // run-time specialised kernels (FP32), one per pass structure
   std::vector<const void*> jk(passes.size(), nullptr);
@@ -1256,7 +1287,9 @@ static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& pa
           rb = kRegBits;
           sp = SerialPlan();
           if (accs) accs->resize(accs0);
-          serialize_plan<R, M, ADJ>(n, h->dtype, passes, sp, accs, packed, rb);
+          passes = std::move(plain);
+          if (defer) *defer = *before;
+          serialize_plan<R, M, ADJ>(n, h->dtype, passes, sp, accs, defer, packed, rb);
           jk.assign(passes.size(), nullptr);
           compile();
         }
@@ -1396,11 +1429,13 @@ static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const do
       return analyze_gate(h->nq, gates[bad[t]].nq, gates[bad[t]].pos, mats + gates[bad[t]].mat, false, specs[bad[t]]);
   std::vector<PlanPass> passes;
   plan_passes(h->nq, tile_config(h->dtype, h->nq), false, items, passes);
-  if (defer && (use_packed(h) || plans_like_jit64(h))) defer_phases(h->nq, false, h->dtype == VQC_C64, passes);
+  std::optional<Deferred> deferred;
+  if (defer && (use_packed(h) || plans_like_jit64(h))) deferred.emplace(h->nq, false, h->dtype == VQC_C64, passes);
+  Deferred* df = deferred ? &*deferred : nullptr;
   const uint64_t call = new_call();
   const char* pc = std::getenv("VQC_PLAN_CHUNKS");  // 0: one serialisation for the whole sweep
   if (passes.size() < 4 || (pc && *pc && std::atoi(pc) == 0))
-    return run_plan<R, M, false>(h, h->d, nullptr, passes, specs, nullptr, nullptr, call);
+    return run_plan<R, M, false>(h, h->d, nullptr, passes, specs, nullptr, nullptr, call, df);
   // Serialised and launched in chunks of 1, 2, 4, ... passes: the host plans
   // the next chunk while the device runs the previous ones, instead of the
   // device waiting for the whole sweep's descriptors (about 1.5 ms for 2,000
@@ -1416,7 +1451,7 @@ static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const do
     std::vector<PlanPass> chunk(std::make_move_iterator(passes.begin() + first),
                                 std::make_move_iterator(passes.begin() + last));
     size_t used = 0;
-    if ((rc = run_plan<R, M, false>(h, h->d, nullptr, chunk, specs, nullptr, nullptr, call, off, &used))) return rc;
+    if ((rc = run_plan<R, M, false>(h, h->d, nullptr, chunk, specs, nullptr, nullptr, call, df, off, &used))) return rc;
     off = (off + used + 255) & ~size_t(255);
   }
   return VQC_OK;
@@ -1489,7 +1524,9 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
   std::vector<PItem> items = reverse_items(specs, params);
   std::vector<PlanPass> passes;
   plan_passes(h->nq, tile_config(h->dtype, h->nq), true, items, passes);
-  if (use_packed(h) || plans_like_jit64(h)) defer_phases(h->nq, true, h->dtype == VQC_C64, passes);
+  std::optional<Deferred> deferred;
+  if ((use_packed(h) || plans_like_jit64(h)) && Deferred::applies(true, passes))
+    deferred.emplace(h->nq, true, h->dtype == VQC_C64, passes);
   // standalone gates with parameters: split their passes out so the per-gate
   // path can evaluate the partials right after the uncompute
   std::vector<AccRef> accs;
@@ -1540,7 +1577,8 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
     take *= 2;
     std::vector<AccRef> gaccs;
     size_t used = 0;
-    int rc = run_plan<R, M, true>(h, y, lam, group, specs, &gaccs, h->accbuf + (size_t)row_base * 8, call, off, &used);
+    int rc = run_plan<R, M, true>(h, y, lam, group, specs, &gaccs, h->accbuf + (size_t)row_base * 8, call,
+                                   deferred ? &*deferred : nullptr, off, &used);
     if (rc) return rc;
     off = (off + used + 255) & ~size_t(255);
     for (auto& a : gaccs) {
@@ -1644,8 +1682,9 @@ static int build_plan_tm(int n, int dtype, const std::vector<GateSpec>& fspecs, 
   plan_passes(n, tc, false, items, passes);
   for (const PlanPass& p : passes)
     if (p.standalone) return fail(VQC_ERR_UNSUPPORTED, "serving takes gates with at most two target qubits");
-  if (packed) defer_phases(n, false, dtype == VQC_C64, passes);
-  serialize_plan<R, M, false>(n, dtype, passes, rp.fwd, nullptr, packed);
+  std::optional<Deferred> deferred;
+  if (packed) deferred.emplace(n, false, dtype == VQC_C64, passes);
+  serialize_plan<R, M, false>(n, dtype, passes, rp.fwd, nullptr, deferred ? &*deferred : nullptr, packed);
   rp.fwd_max = shape_max(rp.fwd);
   if (want_grad) {
     std::vector<PItem> ritems = reverse_items(rspecs, params);
@@ -1654,8 +1693,8 @@ static int build_plan_tm(int n, int dtype, const std::vector<GateSpec>& fspecs, 
     for (const PlanPass& p : rpasses)
       if (p.standalone)
         return fail(VQC_ERR_UNSUPPORTED, "serving takes parameterised gates with one target qubit (or diagonal)");
-    if (packed) defer_phases(n, true, dtype == VQC_C64, rpasses);
-    serialize_plan<R, M, true>(n, dtype, rpasses, rp.adj, &rp.accs, packed);
+    if (packed) deferred.emplace(n, true, dtype == VQC_C64, rpasses);
+    serialize_plan<R, M, true>(n, dtype, rpasses, rp.adj, &rp.accs, deferred ? &*deferred : nullptr, packed);
     rp.adj_max = shape_max(rp.adj);
   }
   rp.M = M;

@@ -45,7 +45,8 @@ struct FOp {
   int nd = 0;
   int dq[5] = {0, 0, 0, 0, 0};
   int form = -1;         // U1: a form chosen by its place (kForm*), -1: read off the matrix
-  double gain = 1;       // what executing the op multiplies the state's deferred norm by
+  double norm = 1;       // the state's deferred norm once the op has run (see Deferred)
+  bool later = false;    // U1 without controls: another one follows on its qubit
   bool acc = false;
   std::vector<PGrad> grads;
 };
@@ -60,7 +61,7 @@ struct PassShape {
 struct AccRef {
   int row;
   std::vector<PGrad> grads;
-  double scale = 1;  // of the partials (the deferred norm squared when the op ran)
+  double scale = 1;  // of the partials (the deferred norm squared once the op has run)
   bool ah = false;  // the row holds the anti-Hermitian projection (kAccAH)
 };
 
@@ -83,6 +84,7 @@ struct SerialPlan {
   std::vector<PassLoc> locs;
   size_t pool_off = 0;
   int rows = 0;  // accumulation rows (ADJ)
+  double norm_lo = 1, norm_hi = 1;  // the deferred norm's range over the ops, as they run
 };
 
 
