@@ -299,15 +299,15 @@ static void plan_passes(int n, const TileConfig& tc, bool adj, std::vector<PItem
 // gate outside the tile passes) takes its whole matrix and g, so no pass is added.
 //
 // The amplitudes in flight are the true ones times 1 / |g|, so |g| is bounded: the
-// first deferred gate of a pass and every kNormEvery-th after it take the norm of g
-// (real diagonal, 12 FMAs), and so does one that would take |g| out of the window
-// [kNormMin, 1 / kNormMin].  The gates are walked in the order they run, stage by
+// first deferred gate of a pass and every 8th (FP64: 32nd) after it take the norm of g
+// (real diagonal, 12 FMAs), and so does one that would take |g| out of a window,
+// [1e-12, 1e12] (FP64: 1e-60).  The gates are walked in the order they run, stage by
 // stage: a stage runs every layer of its few register qubits, so in any other order
 // (the planner's, 192 ops to a pass) the factors of one qubit pair's forty layers
 // would meet before the gates meant to take them.  A deferred gate's factor is
 // |cos| of a half angle, one half in the geometric mean: 2^-8 between two norms in
 // FP32, whose reverse sweep sums products of two such amplitudes; the window is
-// reached by chance less than once in 10^5 runs of eight random gates, by gates
+// reached by chance less than twice in 10^5 runs of eight random gates, by gates
 // near X (RX(pi)) at once.
 //
 // Which form a gate takes depends on its place alone, not on its angle (but for
@@ -1574,7 +1574,7 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
     std::vector<PlanPass> group;
     if (jit_compiles() != compiles) take = passes.size();
     while (pj < passes.size() && !passes[pj].standalone && group.size() < take) group.push_back(std::move(passes[pj++]));
-    take *= 2;
+    take = std::min(2 * take, passes.size());  // (a sweep has a chunk per gate outside the passes: doubling is bounded)
     std::vector<AccRef> gaccs;
     size_t used = 0;
     int rc = run_plan<R, M, true>(h, y, lam, group, specs, &gaccs, h->accbuf + (size_t)row_base * 8, call,
