@@ -141,8 +141,8 @@ struct vqc_state_s {
   void* opbuf = nullptr;       // device buffer for op lists (terms, passes)
   size_t opbuf_bytes = 0;
   void* work[3] = {nullptr, nullptr, nullptr};  // state-sized workspaces (gradients)
-  double* accbuf = nullptr;    // gradient partial sums, one row per parameterised gate
-  size_t accbuf_rows = 0;
+  void* accbuf = nullptr;  // gradient sums, one row of 8 doubles per accumulating op
+  size_t accbuf_bytes = 0;
   void* fused_scratch = nullptr;  // per-CTA partial sums of the tile engine
   size_t fused_scratch_bytes = 0;
   void* outbuf = nullptr;  // results on their way to the host (partial trace, probabilities)
@@ -165,9 +165,26 @@ int workspace(vqc_state h, int count, void** bufs);
 int enter(vqc_state h);
 // Device memory of handles.  dev_free keeps buffers for later handles (at most
 // kPoolBytes per device; all are given back when the device's last handle goes
-// or an allocation fails); every use of a buffer must have completed.
+// or an allocation of this library fails); every use of a buffer must have
+// completed.
 int dev_alloc(int device, void** p, size_t bytes);
 void dev_free(int device, void* p, size_t bytes);
+// Gives the kept memory back to the driver.
+void dev_give_back(int device);
+// Runs `alloc` (a CUDA allocation), and once more without the kept memory if
+// the device had none left.
+template <class F>
+cudaError_t alloc_retry(int device, F alloc) {
+  cudaError_t e = alloc();
+  if (e != cudaErrorMemoryAllocation) return e;
+  dev_give_back(device);
+  e = alloc();
+  cudaGetLastError();  // (a failed allocation's error must not be read as a later launch's)
+  return e;
+}
+// Grows a handle's buffer *buf of *have bytes to at least `need`: after its
+// stream has drained, to a power of two (the next handle's are then the same).
+int reserve_buffer(vqc_state h, void** buf, size_t* have, size_t need);
 // Grows h->opbuf to at least `bytes` and copies `src` into it (stream-ordered).
 int upload_ops(vqc_state h, const void* src, size_t bytes);
 int reserve_ops(vqc_state h, size_t bytes);

@@ -1333,15 +1333,7 @@ static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& pa
     }
   double* partials = nullptr;
   if (ADJ && need > 0) {
-    if (need > h->fused_scratch_bytes) {
-      if (h->fused_scratch) {
-        VQC_CK(cudaStreamSynchronize(h->stream));
-        VQC_CK(cudaFree(h->fused_scratch));
-        h->fused_scratch = nullptr;
-      }
-      VQC_CK(cudaMalloc(&h->fused_scratch, need));
-      h->fused_scratch_bytes = need;
-    }
+    if (int rc = reserve_buffer(h, &h->fused_scratch, &h->fused_scratch_bytes, need)) return rc;
     partials = (double*)h->fused_scratch;
   }
   // the reduction items travel with the pass descriptors
@@ -1537,16 +1529,7 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
       for (auto& f : p.ops) s += f.acc ? 1 : 0;
       total_rows += s;
     }
-  if ((size_t)total_rows * 8 > h->accbuf_rows * 32) {
-    if (h->accbuf) {
-      VQC_CK(cudaStreamSynchronize(h->stream));
-      VQC_CK(cudaFree(h->accbuf));
-      h->accbuf = nullptr;
-    }
-    const size_t rows32 = ((size_t)total_rows * 8 + 31) / 32 + 1;
-    VQC_CK(cudaMalloc(&h->accbuf, sizeof(double) * 32 * rows32));
-    h->accbuf_rows = rows32;
-  }
+  if (int rc = reserve_buffer(h, &h->accbuf, &h->accbuf_bytes, sizeof(double) * 8 * total_rows)) return rc;
   // run pass by pass so that standalone gates with parameters see the right states
   const uint64_t call = new_call();
   int row_base = 0;
@@ -1577,7 +1560,7 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
     take = std::min(2 * take, passes.size());  // (a sweep has a chunk per gate outside the passes: doubling is bounded)
     std::vector<AccRef> gaccs;
     size_t used = 0;
-    int rc = run_plan<R, M, true>(h, y, lam, group, specs, &gaccs, h->accbuf + (size_t)row_base * 8, call,
+    int rc = run_plan<R, M, true>(h, y, lam, group, specs, &gaccs, (double*)h->accbuf + (size_t)row_base * 8, call,
                                    deferred ? &*deferred : nullptr, off, &used);
     if (rc) return rc;
     off = (off + used + 255) & ~size_t(255);

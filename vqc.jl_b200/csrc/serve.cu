@@ -316,7 +316,7 @@ static void worker_main(vqc_server_s* s) {
       }
     }
     for (auto& r : admitted) {
-      SRV_CK(cudaMallocAsync((void**)&r->dmem, r->dbytes, s->stream));
+      SRV_CK(alloc_retry(s->device, [&] { return cudaMallocAsync((void**)&r->dmem, r->dbytes, s->stream); }));
       {
         size_t want = 64;
         while (want < 2 + 8 * (size_t)std::max(r->plan.adj.rows, 1)) want <<= 1;
@@ -447,9 +447,10 @@ static void worker_main(vqc_server_s* s) {
       SRV_CK(cudaStreamSynchronize(s->stream));
       if (s->h_items) cudaFreeHost(s->h_items);
       if (s->d_items) cudaFree(s->d_items);
+      s->h_items = nullptr, s->d_items = nullptr;
       s->items_cap = std::max<size_t>(need * 2, 1 << 16);
-      SRV_CK(cudaMallocHost((void**)&s->h_items, s->items_cap));
-      SRV_CK(cudaMalloc((void**)&s->d_items, s->items_cap));
+      SRV_CK(alloc_retry(s->device, [&] { return cudaMallocHost((void**)&s->h_items, s->items_cap); }));
+      SRV_CK(alloc_retry(s->device, [&] { return cudaMalloc((void**)&s->d_items, s->items_cap); }));
     }
     size_t pos = 0;
     auto put = [&](const void* src, size_t b) {

@@ -91,10 +91,10 @@ void give_back(Pool& p) {  // mu held, the device current
 int new_parts(int device, Parts& q) {
   const int maxb = device_info(device).sms * 8;
   q.scr.max_blocks = maxb;
-  VQC_CK(cudaMalloc(&q.scr.partials, sizeof(double) * kMaxAcc * maxb));
-  VQC_CK(cudaMalloc(&q.scr.counter, sizeof(unsigned) * 4));
-  VQC_CK(cudaMalloc(&q.scr.result, sizeof(double) * kMaxAcc));
-  VQC_CK(cudaMallocHost(&q.h_result, sizeof(double) * kMaxAcc));
+  VQC_CK(alloc_retry(device, [&] { return cudaMalloc(&q.scr.partials, sizeof(double) * kMaxAcc * maxb); }));
+  VQC_CK(alloc_retry(device, [&] { return cudaMalloc(&q.scr.counter, sizeof(unsigned) * 4); }));
+  VQC_CK(alloc_retry(device, [&] { return cudaMalloc(&q.scr.result, sizeof(double) * kMaxAcc); }));
+  VQC_CK(alloc_retry(device, [&] { return cudaMallocHost(&q.h_result, sizeof(double) * kMaxAcc); }));
   VQC_CK(cudaStreamCreateWithFlags(&q.stream, cudaStreamNonBlocking));
   return VQC_OK;
 }
@@ -137,13 +137,7 @@ int dev_alloc(int device, void** out, size_t bytes) {
       return VQC_OK;
     }
   }
-  cudaError_t e = cudaMalloc(out, bytes);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    std::lock_guard<std::mutex> lk(p.mu);
-    give_back(p);
-    e = cudaMalloc(out, bytes);
-  }
+  const cudaError_t e = alloc_retry(device, [&] { return cudaMalloc(out, bytes); });
   return e == cudaSuccess ? VQC_OK : cuda_fail(e, "cudaMalloc");
 }
 
@@ -159,20 +153,30 @@ void dev_free(int device, void* buf, size_t bytes) {
   }
 }
 
+void dev_give_back(int device) {
+  Pool& p = pool(device);
+  std::lock_guard<std::mutex> lk(p.mu);
+  give_back(p);
+}
+
+int reserve_buffer(vqc_state h, void** buf, size_t* have, size_t need) {
+  if (need <= *have) return VQC_OK;
+  if (*buf) {
+    VQC_CK(cudaStreamSynchronize(h->stream));
+    VQC_CK(cudaFree(*buf));
+    *buf = nullptr;
+    *have = 0;
+  }
+  size_t cap = 1 << 16;
+  while (cap < need) cap <<= 1;
+  if (int rc = dev_alloc(h->device, buf, cap)) return rc;
+  *have = cap;
+  return VQC_OK;
+}
+
 int upload_ops(vqc_state h, const void* src, size_t bytes) {
   if (bytes == 0) return VQC_OK;
-  if (bytes > h->opbuf_bytes) {
-    if (h->opbuf) {
-      VQC_CK(cudaStreamSynchronize(h->stream));
-      VQC_CK(cudaFree(h->opbuf));
-      h->opbuf = nullptr;
-      h->opbuf_bytes = 0;
-    }
-    size_t cap = 1 << 16;
-    while (cap < bytes) cap <<= 1;
-    if (int rc = dev_alloc(h->device, &h->opbuf, cap)) return rc;
-    h->opbuf_bytes = cap;
-  }
+  if (int rc = reserve_buffer(h, &h->opbuf, &h->opbuf_bytes, bytes)) return rc;
   // Pageable source: the copy is staged before the call returns, so the caller
   // may reuse `src` at once.
   VQC_CK(cudaMemcpyAsync(h->opbuf, src, bytes, cudaMemcpyHostToDevice, h->stream));
@@ -181,20 +185,7 @@ int upload_ops(vqc_state h, const void* src, size_t bytes) {
 
 // The op buffer holds at least `bytes` (a larger buffer replaces it after the
 // stream has drained: call before uploading anything the coming launches read).
-int reserve_ops(vqc_state h, size_t bytes) {
-  if (bytes <= h->opbuf_bytes) return VQC_OK;
-  if (h->opbuf) {
-    VQC_CK(cudaStreamSynchronize(h->stream));
-    VQC_CK(cudaFree(h->opbuf));
-    h->opbuf = nullptr;
-    h->opbuf_bytes = 0;
-  }
-  size_t cap = 1 << 16;
-  while (cap < bytes) cap <<= 1;
-  if (int rc = dev_alloc(h->device, &h->opbuf, cap)) return rc;
-  h->opbuf_bytes = cap;
-  return VQC_OK;
-}
+int reserve_ops(vqc_state h, size_t bytes) { return reserve_buffer(h, &h->opbuf, &h->opbuf_bytes, bytes); }
 
 // Upload into the op buffer at byte offset `off` (reserved with reserve_ops);
 // stream-ordered like upload_ops, so launches queued before it keep reading
@@ -473,8 +464,8 @@ int vqc_state_destroy(vqc_state h) {
   for (void* w : h->work) dev_free(h->device, w, bytes);
   dev_free(h->device, h->opbuf, h->opbuf_bytes);
   dev_free(h->device, h->outbuf, h->outbuf_bytes);
-  if (h->accbuf) cudaFree(h->accbuf);
-  if (h->fused_scratch) cudaFree(h->fused_scratch);
+  dev_free(h->device, h->accbuf, h->accbuf_bytes);
+  dev_free(h->device, h->fused_scratch, h->fused_scratch_bytes);
   Parts q;
   q.stream = h->stream;
   q.scr = h->scr;
