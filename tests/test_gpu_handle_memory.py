@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import vqcb200 as V
-from helpers import max_abs, rand_psi
+from helpers import max_abs, max_rel, rand_psi
 from oracle import oracle as O
 from vqcb200 import workloads as W
 from vqcb200.serve import Server
@@ -90,3 +90,24 @@ def test_serving_takes_the_kept_memory():
         torch.cuda.empty_cache()
     assert abs(e - e_ref) <= 1e-5 * abs(e_ref) and np.linalg.norm(g - g_ref) <= 1e-5 * np.linalg.norm(g_ref)
     assert len(keep.storage()) == 16
+
+
+@pytest.mark.parametrize("n,kept", [(9, True), (13, False)])
+def test_a_large_partial_trace_leaves_nothing_on_its_handle(n, kept):
+    """One qubit traced out of 13 is 256 MiB of result: it goes back with the call, and the handle's next
+    allocation finds it (the second trace of the same size takes no more)."""
+    rng = np.random.default_rng(960)
+    psi = rand_psi(rng, n)
+    rho = V.DensityMatrix(V.StateVector(psi.astype(np.complex64), dtype=np.complex64))
+    m = psi.astype(np.complex64).astype(np.complex128).reshape(-1, 2)  # (the row's low bit is qubit 1)
+    for _ in range(2):
+        assert max_rel(V.partial_tr(rho, [1]), m @ m.conj().T) < 1e-5
+    if kept:
+        return
+    with pytest.raises(Exception):
+        V.StateVector(36, dtype=np.complex64)  # gives the kept memory back
+    before = free_bytes()
+    V.partial_tr(rho, [1])
+    with pytest.raises(Exception):
+        V.StateVector(36, dtype=np.complex64)
+    assert before - free_bytes() < 64 * MB

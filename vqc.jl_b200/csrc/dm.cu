@@ -58,22 +58,36 @@ int dm_apply_gate_raw(vqc_state h, int k, const int* pos, const double* mat) {
   return apply_gate_raw(h, k, p2, Uc.data());
 }
 
-// The handle's buffer of results for the host, kept between calls: a
-// stream-ordered allocation per call gave its memory back to the driver at every
-// synchronisation (12 qubits: partial trace 1.87 -> 0.84 ms, probabilities 576 ->
-// 35 us).
-static int reserve_out(vqc_state h, size_t bytes) {
-  if (bytes <= h->outbuf_bytes) return VQC_OK;
-  if (h->outbuf) {
-    VQC_CK(cudaStreamSynchronize(h->stream));
-    VQC_CK(cudaFree(h->outbuf));
-    h->outbuf = nullptr;
-    h->outbuf_bytes = 0;
+// Device memory for results on their way to the host.  Up to kOutBytes the handle
+// keeps its buffer between calls: a stream-ordered allocation per call gave its
+// memory back to the driver at every synchronisation (12 qubits: partial trace
+// 1.87 -> 0.84 ms, probabilities 576 -> 35 us).  A larger one ends with the call (one
+// qubit traced out of 15 in FP64 is 4 GiB, a quarter of the state).
+constexpr size_t kOutBytes = size_t(64) << 20;
+struct OutBuffer {
+  explicit OutBuffer(vqc_state s) : h(s) {}
+  OutBuffer(const OutBuffer&) = delete;
+  OutBuffer& operator=(const OutBuffer&) = delete;
+  ~OutBuffer() {
+    if (!own) return;
+    cudaStreamSynchronize(h->stream);  // (a failed call may leave work on it)
+    dev_free(h->device, own, bytes);
   }
-  if (int rc = dev_alloc(h->device, &h->outbuf, bytes)) return rc;
-  h->outbuf_bytes = bytes;
-  return VQC_OK;
-}
+  int reserve(size_t want, void** p) {
+    if (want <= kOutBytes) {
+      const int rc = reserve_buffer(h, &h->outbuf, &h->outbuf_bytes, want);
+      *p = h->outbuf;
+      return rc;
+    }
+    bytes = want;
+    const int rc = dev_alloc(h->device, &own, want);
+    *p = own;
+    return rc;
+  }
+  vqc_state h;
+  void* own = nullptr;
+  size_t bytes = 0;
+};
 
 // rho[r + L c] = psi[r] conj(psi[c])
 template <class R>
@@ -379,8 +393,9 @@ int vqc_dm_ptrace(vqc_state rho, int nsites, const int* sites, double* out) {
   const int nk = n - nsites;
   const int64_t s1 = int64_t(1) << nk;
   std::lock_guard<std::mutex> lk(rho->mu);
-  if ((rc = reserve_out(rho, sizeof(double2) * s1 * s1))) return rc;
-  double2* dout = (double2*)rho->outbuf;
+  OutBuffer buf(rho);
+  double2* dout = nullptr;
+  if ((rc = buf.reserve(sizeof(double2) * s1 * s1, (void**)&dout))) return rc;
   const int g = launch_grid(rho->device, s1 * s1);
   if (rho->dtype == VQC_C64)
     k_dm_ptrace<float><<<g, 256, 0, rho->stream>>>((const float2*)rho->d, n, kept, traced, nk, nsites, dout);
@@ -402,8 +417,9 @@ int vqc_dm_probs(vqc_state rho, double* out) {
   if (!out) return fail(VQC_ERR_ARG, "null output");
   std::lock_guard<std::mutex> lk(rho->mu);
   const int64_t L = int64_t(1) << n;
-  if ((rc = reserve_out(rho, sizeof(double) * L))) return rc;
-  double* dout = (double*)rho->outbuf;
+  OutBuffer buf(rho);
+  double* dout = nullptr;
+  if ((rc = buf.reserve(sizeof(double) * L, (void**)&dout))) return rc;
   const int g = launch_grid(rho->device, L);
   if (rho->dtype == VQC_C64)
     k_dm_diag<float><<<g, 256, 0, rho->stream>>>((const float2*)rho->d, n, dout);
