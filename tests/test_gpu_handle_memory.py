@@ -12,6 +12,7 @@ import pytest
 import vqcb200 as V
 from helpers import max_abs, max_rel, rand_psi
 from oracle import oracle as O
+from vqcb200 import _lib
 from vqcb200 import workloads as W
 from vqcb200.serve import Server
 
@@ -111,3 +112,18 @@ def test_a_large_partial_trace_leaves_nothing_on_its_handle(n, kept):
     with pytest.raises(Exception):
         V.StateVector(36, dtype=np.complex64)
     assert before - free_bytes() < 64 * MB
+
+
+def test_the_first_gradient_of_a_handle_sizes_its_buffers_once(monkeypatch):
+    """Descriptors (forward, reverse), sums, rows: one growth each, not one for every chunk of the sweep."""
+    monkeypatch.setenv("VQC_JIT", "interp")
+    n, layers, rng = 18, 20, np.random.default_rng(970)
+    c = W.to_circuit(W.rxyz_crx_spec(n, layers, rng.uniform(0, 6, layers * (4 * n - 1))))
+    H, grown = W.to_operator(W.xxz_spec(n, 0.5)), []
+    psi = V.StateVector(n, dtype=np.complex64)
+    for _ in range(2):
+        _lib.profile_enable(True)
+        V.energy_and_gradient(H, c, psi)
+        _lib.profile_enable(False)
+        grown.append(_lib.profile_read().get("handle_buffer_grown", (0,))[0])
+    assert 0 < grown[0] <= 4 and grown[1] == 0

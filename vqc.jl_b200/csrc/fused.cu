@@ -1393,6 +1393,29 @@ static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& pa
   return VQC_OK;
 }
 
+// Bytes of the reverse sweep's partial sums, an upper bound for its largest chunk
+// (chunks of 1, 2, 4, ... consecutive tile passes, see reverse_impl): a handle's
+// scratch is sized once, before the first chunk.  Grown chunk by chunk it drained
+// the stream and allocated up to six times in the first gradient of a handle.
+template <class R>
+static size_t partials_bound(vqc_state h, int M, const std::vector<PlanPass>& passes) {
+  // resident CTAs: two tiles each
+  const int64_t per_sm = std::max<int64_t>(device_info(h->device).max_smem_optin / (2 * (sizeof(cplx<R>) << M)), 1);
+  const size_t grid = (size_t)std::min<int64_t>(int64_t(1) << (h->nq - M), device_info(h->device).sms * per_sm);
+  size_t most = 0, take = 1;
+  for (size_t i = 0; i < passes.size();) {
+    size_t slots = 0, k = 0;
+    for (; i < passes.size() && !passes[i].standalone && k < take; ++i, ++k)
+      for (const FOp& f : passes[i].ops) slots += f.acc;
+    if (k == 0)
+      ++i;
+    else
+      take = std::min(2 * take, passes.size());
+    most = std::max(most, slots);
+  }
+  return grid * most * 8 * sizeof(double);
+}
+
 int fused_supported(vqc_state h) { return h->nq >= kMinTileBits && h->nq <= 40; }
 
 template <class R, int M>
@@ -1530,13 +1553,13 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
       total_rows += s;
     }
   if (int rc = reserve_buffer(h, &h->accbuf, &h->accbuf_bytes, sizeof(double) * 8 * total_rows)) return rc;
-  // run pass by pass so that standalone gates with parameters see the right states
   const uint64_t call = new_call();
   int row_base = 0;
   const uint64_t compiles = jit_compiles();
   size_t bound = 256, off = 0, take = 1;
   for (const PlanPass& p : passes) bound += op_bytes_bound<R>(p) + sizeof(RedItem) + 256;
   if (int rc = reserve_ops(h, bound)) return rc;
+  if (int rc = reserve_buffer(h, &h->fused_scratch, &h->fused_scratch_bytes, partials_bound<R>(h, M, passes))) return rc;
   for (size_t pi = 0; pi < passes.size(); ++pi) {
     if (passes[pi].standalone) {
       const int gi = passes[pi].gate;

@@ -161,6 +161,7 @@ void dev_give_back(int device) {
 
 int reserve_buffer(vqc_state h, void** buf, size_t* have, size_t need) {
   if (need <= *have) return VQC_OK;
+  prof_note("handle_buffer_grown", 1);
   if (*buf) {
     VQC_CK(cudaStreamSynchronize(h->stream));
     VQC_CK(cudaFree(*buf));
