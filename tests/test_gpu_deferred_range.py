@@ -86,3 +86,16 @@ def test_only_multiples_of_unitaries_are_deferred(dtype, jit, monkeypatch):
             gates.append(V.QuantumGate((q,), a if (q + i) % 4 else a @ np.array([[1, 0.2], [0, 1]])))
         gates += [V.CNOTGate(q, q + 1) for q in range(1, n)]
     assert deferred(lambda: D.check_forward(gates, n, dtype, rng, unitary=False)) > 0
+
+
+@pytest.mark.parametrize("dtype,n,defers", [(np.complex64, 17, False), (np.complex64, 18, True),
+                                            (np.complex128, 20, False), (np.complex128, 22, False),
+                                            (np.complex128, 23, True)])
+def test_deferred_only_where_passes_are_compiled(dtype, n, defers, monkeypatch):
+    """The interpreted passes run whole matrices."""
+    monkeypatch.delenv("VQC_JIT", raising=False)
+    c = V.QCircuit([V.U3Gate(q, 0.3 * q, 0.2, 0.1) for q in (1, 2)] + [V.CNOTGate(1, 2)] +
+                   [V.U3Gate(q, 0.4, 0.2 * q, 0.1) for q in (1, 2)])
+    psi = V.StateVector(n, dtype=dtype)
+    assert (deferred(lambda: V.apply(c, psi)) > 0) == defers
+    assert abs(psi.norm() - 1) < 1e-6

@@ -315,7 +315,7 @@ static void plan_passes(int n, const TileConfig& tc, bool adj, std::vector<PItem
 // passes.  T is a multiple of a unitary whatever |x|: a large x is as accurate as a
 // small one.
 //
-// Only where the passes are compiled (states of 2^18 FP32, 2^20 FP64 amplitudes
+// Only where the passes are compiled (states of 2^18 FP32, 2^23 FP64 amplitudes
 // and more): the interpreted ones are bound by latency, and a CNOT that was a
 // swap of two loads becomes a product (serving's reverse launches 66 -> 81 us).
 // Measured: reverse pass 1,060 -> 957 us and forward 350 -> 325 us at 2^26 FP32,
@@ -1205,19 +1205,17 @@ static bool use_jit(const vqc_state h) {
 // The packed FP32 plan layout: for the compiled passes, or forced with
 // VQC_JIT=interp (the packed interpreter, the compiled kernels' fallback).
 static bool use_packed(const vqc_state h) { return h->dtype == VQC_C64 && (use_jit(h) || jit_mode() == 3); }
-// FP64 states planned for compiled passes (deferred phases): at least 2^20
-// amplitudes (auto), all (on); compiled: at least 2^kCompileQubits64.
-// Smaller states run such plans interpreted: compiling a call's passes takes the
-// host some seconds and saves 2 ms a call at 23 qubits but 0.2 ms at 20, and a
-// stream of different circuits of 20-22 qubits met a compile in most calls (5
-// against 400 requests a second).
+// FP64 passes planned for compiled kernels (deferred phases) and compiled: states of
+// at least 2^kCompileQubits64 amplitudes (auto), all (on).  Compiling a call's passes
+// takes the host some seconds and saves 2 ms a call at 23 qubits but 0.2 ms at 20,
+// and a stream of different circuits of 20-22 qubits met a compile in most calls (5
+// against 400 requests a second).  Smaller states run whole matrices interpreted;
+// deferred phases cost them 5 to 10 % (U3 + CNOT 705 against 655 us at 20 qubits and
+// 1,952 against 1,759 us at 22, an 11-qubit density matrix 1,983 against 1,823 us).
 constexpr int kCompileQubits64 = 23;
-static bool plans_like_jit64(const vqc_state h) {
-  const int mode = jit_mode();
-  return h->dtype == VQC_C128 && (mode == 1 || (mode == 2 && h->nq >= 20)) && jit_available();
-}
 static bool use_jit64(const vqc_state h) {
-  return plans_like_jit64(h) && (jit_mode() == 1 || h->nq >= kCompileQubits64);
+  const int mode = jit_mode();
+  return h->dtype == VQC_C128 && (mode == 1 || (mode == 2 && h->nq >= kCompileQubits64)) && jit_available();
 }
 static uint64_t new_call() {
   static std::atomic<uint64_t> n{0};
@@ -1316,7 +1314,7 @@ static int run_plan(vqc_state h, void* psi, void* lam, std::vector<PlanPass>& pa
                          : kernel_grid(h->device, tile_kernel<R, ADJ>(M, locs[pi].shape), 1 << (M - kRegBits), smem);
     // the CTAs' partial sums group alike in both kernels of an FP64 pass
     if constexpr (ADJ && std::is_same<R, double>::value)
-      if (plans_like_jit64(h)) g = device_info(h->device).sms * jit_min_blocks64(true);
+      if (use_jit64(h)) g = device_info(h->device).sms * jit_min_blocks64(true);
     grids[pi] = (int)std::min<int64_t>(g, locs[pi].ntiles);
   }
   // partial sums scratch: one row of 8 doubles per (CTA, slot) of every pass,
@@ -1445,7 +1443,7 @@ static int forward_impl(vqc_state h, const vqc_gate* gates, int ngates, const do
   std::vector<PlanPass> passes;
   plan_passes(h->nq, tile_config(h->dtype, h->nq), false, items, passes);
   std::optional<Deferred> deferred;
-  if (defer && (use_packed(h) || plans_like_jit64(h))) deferred.emplace(h->nq, false, h->dtype == VQC_C64, passes);
+  if (defer && (use_packed(h) || use_jit64(h))) deferred.emplace(h->nq, false, h->dtype == VQC_C64, passes);
   Deferred* df = deferred ? &*deferred : nullptr;
   const uint64_t call = new_call();
   const char* pc = std::getenv("VQC_PLAN_CHUNKS");  // 0: one serialisation for the whole sweep
@@ -1540,7 +1538,7 @@ static int reverse_impl(vqc_state h, void* lam, void* y, const std::vector<GateS
   std::vector<PlanPass> passes;
   plan_passes(h->nq, tile_config(h->dtype, h->nq), true, items, passes);
   std::optional<Deferred> deferred;
-  if ((use_packed(h) || plans_like_jit64(h)) && Deferred::applies(true, passes))
+  if ((use_packed(h) || use_jit64(h)) && Deferred::applies(true, passes))
     deferred.emplace(h->nq, true, h->dtype == VQC_C64, passes);
   // standalone gates with parameters: split their passes out so the per-gate
   // path can evaluate the partials right after the uncompute
