@@ -716,19 +716,24 @@ int jit_pass_kernels64(int M, bool adj, const std::vector<JitPassRef64>& refs, s
         out[i] = it->second;
       else if (seen64().emplace(keys[i], call).first->second == call && !at_once)
         all_seen = false;
+      else if (inflight().count(keys[i]))
+        continue;  // (another thread compiles it: interpreted this time)
       else if (std::find_if(miss.begin(), miss.end(), [&](size_t m) { return keys[m] == keys[i]; }) == miss.end())
         miss.push_back(i);
     }
+    if (miss.empty() || !all_seen) return VQC_OK;
+    for (size_t m : miss) inflight().insert(keys[m]);
   }
-  if (miss.empty() || !all_seen) return VQC_OK;
   std::vector<std::string> srcs(miss.size());
   for (size_t k = 0; k < miss.size(); ++k) {
     const JitPassRef64& r = refs[miss[k]];
     srcs[k] = jit_pass_source64(M, adj, r.stages, r.nstages, r.ops, r.npool);
   }
   std::vector<const void*> ks;
-  if (int rc = jit_kernels(srcs, ks, "vqc_pass64")) return rc;
+  const int rc = jit_kernels(srcs, ks, "vqc_pass64");
   std::lock_guard<std::mutex> lk(g_mu);
+  for (size_t m : miss) inflight().erase(keys[m]);
+  if (rc) return rc;
   for (size_t k = 0; k < miss.size(); ++k) hcache()[keys[miss[k]]] = ks[k];  // (nullptr: failed; interpreted)
   for (size_t i = 0; i < refs.size(); ++i) {
     auto it = hcache().find(keys[i]);
