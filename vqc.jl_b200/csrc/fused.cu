@@ -721,13 +721,15 @@ static int acc_kind(const FOp& f) {
   return kAccFull;
 }
 // Every D of the op anti-Hermitian (as U^dagger dU/dtheta of a unitary family
-// is): the FP32 body then accumulates the four-value projection (kAccAH).
-static bool acc_anti_hermitian(const FOp& f) {
+// is): four values are then accumulated instead of eight (kAccAH).  rounding: what
+// of D, relative to it, counts as the rounding of U^dagger dU and of the merges.
+constexpr double kRounding32 = 1e-12, kRounding64 = 1e-14;
+static bool acc_anti_hermitian(const FOp& f, double rounding) {
   for (const PGrad& pg : f.grads) {
     if (pg.D.size() != 4) return false;
     double scale = 0;
     for (const cd& d : pg.D) scale = std::max(scale, std::abs(d));
-    const double eps = 1e-12 * scale;
+    const double eps = rounding * scale;
     if (std::abs(pg.D[0].real()) > eps || std::abs(pg.D[3].real()) > eps ||
         std::abs(pg.D[1] + std::conj(pg.D[2])) > eps)
       return false;
@@ -767,7 +769,7 @@ static double pass_fma_ops(const PlanPass& p, int n, bool adj) {
       double o = (double)per_pair[u1_form(f)] * nst;
       if (adj && f.acc) {
         const int k = acc_kind(f);
-        if (acc_anti_hermitian(f))
+        if (acc_anti_hermitian(f, kRounding32))
           o += k == kAccFull ? 12 : (k == kAccOff ? 8 : 4);
         else
           o += k == kAccFull ? 16 : 8;
@@ -904,7 +906,7 @@ static void stage_f32(const PlanPass& p, const PlanStage& st, int M, uint64_t ti
     if (f.kind == kOpU1) {
       const int tb = jbit(tbit[f.tq[0]]), form = u1_form(f);
       o.code |= op_r_bits(tb, 0) | form_bits(form) | (rctl << 16);
-      if (adj && f.acc) o.code |= (acc_kind(f) << 14) | (acc_anti_hermitian(f) ? kCodeAH : 0);
+      if (adj && f.acc) o.code |= (acc_kind(f) << 14) | (acc_anti_hermitian(f, kRounding32) ? kCodeAH : 0);
       const cd u00 = f.mat[0], u01 = f.mat[1], u10 = f.mat[2], u11 = f.mat[3];
       if (tb != 0) {
         switch (form) {
@@ -1066,7 +1068,8 @@ static void serialize_plan(int n, int dtype, std::vector<PlanPass>& passes, Seri
         if (f.kind == kOpU1) {
           const int r = slot_of(tbit[f.tq[0]]), form = interpreted_form<R>(u1_form(f));
           sel = kSelU1 + (r | (rc.n ? 4 : 0) | form << 3);
-          if (ADJ && f.acc) o.code |= (acc_kind(f) << 14) | (acc_anti_hermitian(f) ? kCodeAH : 0);
+          const double rounding = sizeof(R) == 4 ? kRounding32 : kRounding64;
+          if (ADJ && f.acc) o.code |= (acc_kind(f) << 14) | (acc_anti_hermitian(f, rounding) ? kCodeAH : 0);
         }
         if (f.kind == kOpU2) sel = kSelU2 + slot_of(tbit[f.tq[0]]) * 4 + slot_of(tbit[f.tq[1]]);
         if (k0 >= 0) o.code = (o.code & ~15) | kOpPhase;
