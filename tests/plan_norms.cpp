@@ -1,9 +1,11 @@
 // Plans circuits on the host and prints the range of the deferred norm over
-// their passes, in the order the ops run (test_plan_norms.py).
+// their passes, in the order the ops run, the rows of the reverse sweep and a
+// hash of the passes' structure (test_plan_norms.py).
 //   plan_norms <family> <qubits> <layers> <seed>
 // families: blocks2, blocks3 (RZ RY RZ on every qubit, CZ inside blocks, RY a
 // parameter in every tenth layer), pi (RX(pi) rounded to float, CZ brickwork,
-// RX a parameter in every fourth layer), u3 (U3 and CZ brickwork).
+// RX a parameter in every fourth layer), u3 (U3 and CZ brickwork; in every third
+// layer the U3 of one qubit lies next to theta = pi, 1e-8 to 1e-2 off).
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -55,10 +57,17 @@ int main(int argc, char** argv) {
         add({q}, {c, -i * s, -i * s, c});
         if (l % 4 == 1) param({-s / 2, -i * c / 2.0, -i * c / 2.0, -s / 2});
       } else {
-        const double t = angle() / 2, c = std::cos(t), s = std::sin(t);
+        double t = angle() / 2;
+        if (fam == "u3") {
+          if (l % 3 == 0 && q == (5 * l + 3) % n) t = M_PI / 2 - std::pow(10.0, -2 - 6 * t / M_PI);
+          const double c = std::cos(t), s = std::sin(t), p = angle(), m = angle();
+          add({q}, {c, -std::polar(s, m), std::polar(s, p), std::polar(c, p + m)});
+          continue;
+        }
+        const double c = std::cos(t), s = std::sin(t);
         rz(q);
         add({q}, {c, -s, s, c});
-        if (fam != "u3" && l % 10 == 5) param({-s / 2, -c / 2, c / 2, -s / 2});
+        if (l % 10 == 5) param({-s / 2, -c / 2, c / 2, -s / 2});
         rz(q);
       }
     }
@@ -81,6 +90,13 @@ int main(int argc, char** argv) {
   lo = std::min(lo, std::min(packed.fwd.norm_lo, packed.adj.norm_lo));
   hi = std::max(hi, std::max(packed.fwd.norm_hi, packed.adj.norm_hi));
 #endif
-  std::printf("%.6e %.6e %zu\n", lo, hi, packed.accs.size());
+  uint64_t hash = 1469598103934665603ull;
+  for (const SerialPlan* sp : {&packed.fwd, &packed.adj})
+    for (const PassLoc& l : sp->locs) {
+      const DevOp* ops = (const DevOp*)(sp->buf.data() + l.ops);
+      for (int o = 0; o < l.shape.nops; ++o)
+        for (int v : {ops[o].code, ops[o].mat, ops[o].rmask}) hash = (hash ^ (uint32_t)v) * 1099511628211ull;
+    }
+  std::printf("%.6e %.6e %zu %016llx\n", lo, hi, packed.accs.size(), (unsigned long long)hash);
   return 0;
 }

@@ -8,6 +8,7 @@ helpers.py.
 import numpy as np
 import pytest
 
+import test_gpu_pass_memory as crowded
 import vqcb200 as V
 from helpers import as_input, max_abs, rand_psi, rel, tol
 from oracle import oracle as O
@@ -32,3 +33,10 @@ def test_smallest_passes(name, dtype, n, jit, monkeypatch):
     _, g, yin = V.back_propagate(V.StateVector(target.astype(dtype), dtype=dtype), c, y)
     assert max_abs(yin.storage(), psi0) < tol(dtype)
     assert len(g) == len(g_ref) and (len(g) == 0 or rel(g, g_ref) < tol(dtype))
+
+
+@pytest.mark.parametrize("kind", ["pairs", "diagonals"])
+def test_crowded_packed_passes(kind, monkeypatch):
+    """The other end, on the FP32 packed plan: up to 192 ops in a pass, 76 stages, 191 KB of shared memory."""
+    monkeypatch.setenv("VQC_JIT", "interp")
+    crowded.test_crowded_passes(np.complex64, 18, kind)

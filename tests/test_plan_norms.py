@@ -41,6 +41,18 @@ def test_norm_stays_in_the_window(plan_norms, family, n, layers):
         if r.returncode == 3:
             pytest.skip("no run-time compiler: nothing is deferred")
         assert r.returncode == 0, r.stderr
-        lo, hi, rows = r.stdout.split()
+        lo, hi, rows, _ = r.stdout.split()
         assert 1e-12 <= float(lo) < 1 and float(hi) <= 1e12
         assert family == "u3" or int(rows) > 0
+
+
+@pytest.mark.parametrize("family,n,layers,seeds", [("u3", 18, 8, 40), ("u3", 20, 4, 20), ("blocks2", 18, 6, 20)])
+def test_angles_do_not_change_the_structure(plan_norms, family, n, layers, seeds):
+    """Compiled passes are reused for new angles, those with a tiny diagonal included."""
+    found = set()
+    for seed in range(seeds):
+        r = subprocess.run([plan_norms, family, str(n), str(layers), str(seed)], capture_output=True, text=True)
+        if r.returncode == 3:
+            pytest.skip("no run-time compiler: nothing is deferred")
+        found.add(r.stdout.split()[3])
+    assert len(found) == 1

@@ -420,7 +420,7 @@ class Deferred {
         e0 *= d, e3 *= d, e1 *= std::polar(1.0L, -r * cc / 2);
         x = e1 * std::conj(e0) * (s / c);
       }
-      if (std::abs(r) * s <= tol_ * top) {
+      if (std::abs(r) * c * s <= tol_ * top * top) {  // (what it changes of M's entries; a small c has a loose phase)
         p = whole_turns(e3 * std::conj(e0));
         g_ *= e0 * c;
         const bool whole = since_ >= every_ || ng < min_ || ng > 1 / min_;
