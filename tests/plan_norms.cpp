@@ -1,6 +1,7 @@
-// Plans circuits on the host and prints the range of the deferred norm over
-// their passes, in the order the ops run, the rows of the reverse sweep and a
-// hash of the passes' structure (test_plan_norms.py).
+// Plans circuits on the host and prints the range of the deferred norm over the
+// passes of the forward and of the reverse sweep, in the order the ops run, the
+// rows of the reverse sweep and a hash of the passes' structure
+// (test_plan_norms.py).
 //   plan_norms <family> <qubits> <layers> <seed>
 // families: blocks2, blocks3 (RZ RY RZ on every qubit, CZ inside blocks, RY a
 // parameter in every tenth layer), pi (RX(pi) rounded to float, CZ brickwork,
@@ -86,10 +87,7 @@ int main(int argc, char** argv) {
   if (packed.fwd.locs.empty()) return 3;  // (no run-time compiler here: nothing is deferred)
   double lo = 1, hi = 1;
   for (const AccRef& a : packed.accs) lo = std::min(lo, std::sqrt(a.scale)), hi = std::max(hi, std::sqrt(a.scale));
-#ifndef ROWS_ONLY
-  lo = std::min(lo, std::min(packed.fwd.norm_lo, packed.adj.norm_lo));
-  hi = std::max(hi, std::max(packed.fwd.norm_hi, packed.adj.norm_hi));
-#endif
+  lo = std::min(lo, packed.adj.norm_lo), hi = std::max(hi, packed.adj.norm_hi);
   uint64_t hash = 1469598103934665603ull;
   for (const SerialPlan* sp : {&packed.fwd, &packed.adj})
     for (const PassLoc& l : sp->locs) {
@@ -97,6 +95,7 @@ int main(int argc, char** argv) {
       for (int o = 0; o < l.shape.nops; ++o)
         for (int v : {ops[o].code, ops[o].mat, ops[o].rmask}) hash = (hash ^ (uint32_t)v) * 1099511628211ull;
     }
-  std::printf("%.6e %.6e %zu %016llx\n", lo, hi, packed.accs.size(), (unsigned long long)hash);
+  std::printf("%.6e %.6e %.6e %.6e %zu %016llx\n", packed.fwd.norm_lo, packed.fwd.norm_hi, lo, hi, packed.accs.size(),
+              (unsigned long long)hash);
   return 0;
 }

@@ -2,8 +2,8 @@
 
 The planner itself runs (plan_norms.cpp, linked against the engine's library):
 over every op of a sweep, in the order the passes run them, the deferred norm
-must stay inside the window the planner states for FP32, [1e-12, 1e12].  The
-families are those that leave it when the gates are walked in any other order:
+must stay inside the window the planner states for FP32, [1e-12, 1e12] in the
+reverse sweep and [1e-18, 1e18] in the forward one.  The families are those that leave it when the gates are walked in any other order:
 qubits that meet in small blocks only, so that one stage runs all their layers,
 and rotations next to pi, whose diagonal is tiny.
 """
@@ -41,7 +41,8 @@ def test_norm_stays_in_the_window(plan_norms, family, n, layers):
         if r.returncode == 3:
             pytest.skip("no run-time compiler: nothing is deferred")
         assert r.returncode == 0, r.stderr
-        lo, hi, rows, _ = r.stdout.split()
+        fwd_lo, fwd_hi, lo, hi, rows, _ = r.stdout.split()
+        assert 1e-18 <= float(fwd_lo) < 1 and float(fwd_hi) <= 1e18
         assert 1e-12 <= float(lo) < 1 and float(hi) <= 1e12
         assert family == "u3" or int(rows) > 0
 
@@ -54,5 +55,5 @@ def test_angles_do_not_change_the_structure(plan_norms, family, n, layers, seeds
         r = subprocess.run([plan_norms, family, str(n), str(layers), str(seed)], capture_output=True, text=True)
         if r.returncode == 3:
             pytest.skip("no run-time compiler: nothing is deferred")
-        found.add(r.stdout.split()[3])
+        found.add(r.stdout.split()[5])
     assert len(found) == 1

@@ -299,16 +299,17 @@ static void plan_passes(int n, const TileConfig& tc, bool adj, std::vector<PItem
 // gate outside the tile passes) takes its whole matrix and g, so no pass is added.
 //
 // The amplitudes in flight are the true ones times 1 / |g|, so |g| is bounded: the
-// first deferred gate of a pass and every 8th (FP64: 32nd) after it take the norm of g
-// (real diagonal, 12 FMAs), and so does one that would take |g| out of a window,
-// [1e-12, 1e12] (FP64: 1e-60).  The gates are walked in the order they run, stage by
+// first deferred gate of a pass and every 8th after it (forward 16th, FP64 32nd) take
+// the norm of g (real diagonal, 12 FMAs), and so does one that would take |g| out of
+// a window, [1e-12, 1e12] (forward 1e-18, FP64 1e-60).  The gates are walked in the order they run, stage by
 // stage: a stage runs every layer of its few register qubits, so in any other order
 // (the planner's, 192 ops to a pass) the factors of one qubit pair's forty layers
 // would meet before the gates meant to take them.  A deferred gate's factor is
 // |cos| of a half angle, one half in the geometric mean: 2^-8 between two norms in
-// FP32, whose reverse sweep sums products of two such amplitudes; the window is
-// reached by chance less than twice in 10^5 runs of eight random gates, by gates
-// near X (RX(pi)) at once.
+// the FP32 reverse sweep, which sums products of two such amplitudes, 2^-16 in the
+// forward one (every 8th there: 64.0 against 63.2 ms for the 30-qubit circuit); the
+// window is reached by chance less than twice in 10^5 such runs of random gates, by
+// gates near X (RX(pi)) at once.
 //
 // Which form a gate takes depends on its place alone, not on its angle (but for
 // the window, |m00| < kMinPivot and exact zeros), so that new angles reuse compiled
@@ -340,7 +341,8 @@ class Deferred {
  public:
   // Marks the ops of the sweep that a later uncontrolled one-qubit op on their qubit follows.
   Deferred(int n, bool adj, bool f32, std::vector<PlanPass>& passes)
-      : adj_(adj), f32_(f32), every_(f32 ? 8 : 32), min_(f32 ? 1e-12 : 1e-60), tol_(f32 ? 1e-13 : 1e-14),
+      : adj_(adj), f32_(f32), every_(!f32 ? 32 : (adj ? 8 : 16)), min_(!f32 ? 1e-60 : (adj ? 1e-12 : 1e-18)),
+        tol_(f32 ? 1e-13 : 1e-14),
         least_(f32 ? 1e-30 : 1e-280), ph_(n, cl(1)) {
     std::vector<char> open(n, 0);
     for (size_t pi = passes.size(); pi-- > 0;) {
@@ -372,84 +374,103 @@ class Deferred {
   }
 
  private:
+  // (plain products and norms: the library's test for infinities and take hypot,
+  // a microsecond per gate; a long double holds the square of any matrix entry)
+  static cl mul(const cl& a, const cl& b) {
+    return cl(a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real());
+  }
+  static cl mulc(const cl& a, const cl& b) {  // a conj(b)
+    return cl(a.real() * b.real() + a.imag() * b.imag(), a.imag() * b.real() - a.real() * b.imag());
+  }
+  static long double mod(const cl& a) { return std::sqrt(a.real() * a.real() + a.imag() * a.imag()); }
+
   void op(FOp& f) {
     Mat& m = f.mat;
+    const cl one(1);
     if (f.kind == kOpU2) {
       const cl a = ph_[f.tq[0]], b = ph_[f.tq[1]];
-      if (a != cl(1) || b != cl(1)) {
-        const cl c[4] = {cl(1), a, b, a * b};
+      if (a != one || b != one) {
+        const cl c[4] = {one, a, b, mul(a, b)};
         for (int r = 0; r < 4; ++r)
           for (int q = 0; q < 4; ++q)
-            if (m[4 * r + q] != cd(0)) m[4 * r + q] = cd(cl(m[4 * r + q]) * c[q] * std::conj(c[r]));
+            if (m[4 * r + q] != cd(0)) m[4 * r + q] = cd(mulc(mul(cl(m[4 * r + q]), c[q]), c[r]));
       }
     } else if (f.kind == kOpU1 && f.cmask) {
       const cl p = ph_[f.tq[0]];
-      if (p != cl(1)) {
-        if (m[1] != cd(0)) m[1] = cd(cl(m[1]) * p);
-        if (m[2] != cd(0)) m[2] = cd(cl(m[2]) * std::conj(p));
+      if (p != one) {
+        if (m[1] != cd(0)) m[1] = cd(mul(cl(m[1]), p));
+        if (m[2] != cd(0)) m[2] = cd(mulc(cl(m[2]), p));
       }
     } else if (f.kind == kOpU1) {
       one_qubit(f);
     }
-    f.norm = (double)std::abs(g_);
+    f.norm = (double)ng_;
     if (adj_ && f.acc && f.kind == kOpU1) {  // the reduced matrix's frame
       const cl p = ph_[f.tq[0]];
-      if (p != cl(1))
-        for (PGrad& pg : f.grads) pg.D[1] = cd(cl(pg.D[1]) * p), pg.D[2] = cd(cl(pg.D[2]) * std::conj(p));
+      if (p != one)
+        for (PGrad& pg : f.grads) pg.D[1] = cd(mul(cl(pg.D[1]), p)), pg.D[2] = cd(mulc(cl(pg.D[2]), p));
     }
   }
   void one_qubit(FOp& f) {
     cl& p = ph_[f.tq[0]];
-    const cl m0(f.mat[0]), m1 = cl(f.mat[1]) * p, m2(f.mat[2]), m3 = cl(f.mat[3]) * p;
-    const long double n0 = std::abs(m0), n1 = std::abs(m1), n2 = std::abs(m2), n3 = std::abs(m3);
+    const cl m0(f.mat[0]), m1 = mul(cl(f.mat[1]), p), m2(f.mat[2]), m3 = mul(cl(f.mat[3]), p);
+    const long double n0 = mod(m0), n1 = mod(m1), n2 = mod(m2), n3 = mod(m3);
     const long double top = std::max(std::max(n0, n3), std::max(n1, n2));
-    const long double c = (n0 + n3) / 2, s = (n1 + n2) / 2, ng = std::abs(g_) * c;
+    const long double c = (n0 + n3) / 2, s = (n1 + n2) / 2, ng = ng_ * c;
     if (f.later && std::min(n0, n3) > kMinPivot * top && std::abs(n0 - n3) <= tol_ * top &&
         std::abs(n1 - n2) <= tol_ * top && ng > least_ && ng < 1 / least_) {
       // The unitary nearest to M / |.|: the entries' phases, of moduli c, s, s, c,
       // satisfy arg m1 + arg m2 = arg m0 + arg m3 + pi but for the rounding r of the
       // matrix, which is shared out (taking any three entries as they are would put
-      // all of it into the fourth)
+      // all of it into the fourth); r is below 1e-4 where the gate qualifies, so the
+      // angle is its sine and the turn by d is 1 - d^2 / 2 + i d
       cl e0 = m0 / n0, e3 = m3 / n3, x(0);
       long double r = 0;
+      bool unitary = true;
       if (n1 > 0 && n2 > 0) {
         cl e1 = m1 / n1;
-        r = std::arg(-e1 * (m2 / n2) * std::conj(e0 * e3));
-        const long double cc = c * c / (c * c + s * s);
-        const cl d = std::polar(1.0L, r * (1 - cc) / 2);
-        e0 *= d, e3 *= d, e1 *= std::polar(1.0L, -r * cc / 2);
-        x = e1 * std::conj(e0) * (s / c);
+        const cl z = mulc(mul(e1, m2 / n2), mul(e0, e3));
+        r = -z.imag();
+        // (what r changes of M's entries; a small c has a loose phase)
+        unitary = z.real() < 0 && std::abs(r) < 1e-4L && std::abs(r) * c * s <= tol_ * top * top;
+        const long double cc = c * c / (c * c + s * s), d0 = r * (1 - cc) / 2, d1 = -r * cc / 2;
+        const cl t0(1 - d0 * d0 / 2, d0);
+        e0 = mul(e0, t0), e3 = mul(e3, t0), e1 = mul(e1, cl(1 - d1 * d1 / 2, d1));
+        x = mulc(e1, e0) * (s / c);
       }
-      if (std::abs(r) * c * s <= tol_ * top * top) {  // (what it changes of M's entries; a small c has a loose phase)
-        p = whole_turns(e3 * std::conj(e0));
-        g_ *= e0 * c;
+      if (unitary) {
+        p = whole_turns(mulc(e3, e0));
         const bool whole = since_ >= every_ || ng < min_ || ng > 1 / min_;
         const long double d = whole ? rounded(ng) : 1.0L;
         const cl w(rounded(d * x.real()), rounded(d * x.imag()));
-        g_ *= std::sqrt((1 + std::norm(x)) / (1 + std::norm(w / d))) / d;
+        const long double turn = c * std::sqrt((1 + std::norm(x)) / (1 + std::norm(w / d))) / d;
+        g_ = mul(g_, e0) * turn;
+        ng_ *= turn;
         since_ = whole ? 0 : since_ + 1;
         f.form = whole ? kFormRC : (w == cl(0) ? kFormId : kFormUD);
         f.mat = {cd(d), cd(w), -std::conj(cd(w)), cd(d)};
         return;
       }
     }
-    f.mat = {cd(m0 * g_), cd(m1 * g_), cd(m2 * g_), cd(m3 * g_)};
+    f.mat = {cd(mul(m0, g_)), cd(mul(m1, g_)), cd(mul(m2, g_)), cd(mul(m3, g_))};
     g_ = cl(1);
+    ng_ = 1;
     p = cl(1);
   }
   long double rounded(long double v) const { return f32_ ? (long double)(float)v : (long double)(double)v; }
   // A phase within rounding of 1, i, -1 or -i is that one (a rounding error must
   // not decide which form the next gates take).
-  cl whole_turns(cl p) const {
-    for (const cl& q : {cl(1), cl(-1), cl(0, 1), cl(0, -1)})
-      if (std::abs(p - q) < tol_ / 10) return q;
+  cl whole_turns(const cl& p) const {
+    if (std::abs(p.imag()) < tol_ / 10) return cl(p.real() > 0 ? 1 : -1);
+    if (std::abs(p.real()) < tol_ / 10) return cl(0, p.imag() > 0 ? 1 : -1);
     return p;
   }
   bool adj_, f32_;
   int every_, since_ = 0;
   long double min_, tol_, least_;  // (least_: a norm a matrix entry can hold)
   std::vector<cl> ph_;
-  cl g_ = cl(1);
+  cl g_ = cl(1);          // the deferred factor,
+  long double ng_ = 1;    // its norm
 };
 
 // Conflict check of a register-bit set for the shared-memory swizzle.
